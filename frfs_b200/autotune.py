@@ -22,7 +22,8 @@ _CACHE = os.environ.get('BDGFS_TUNE_CACHE',
 
 def _key(grids, nsm):
     parts = [f"{'f64' if g.dtype == torch.float64 else 'f32'}-{g.Nv}-{g.Nrho}-{g.M}" for g in grids]
-    return '|'.join(parts) + f'|sm{nsm}'
+    # the variant count: a cache written by another build does not hide new variants
+    return '|'.join(parts) + f'|sm{nsm}|v{len(variants(grids))}'
 
 
 def _load():

@@ -33,6 +33,7 @@
 // the x-pencil (y,z) in the last pass), Gh accumulates in per-CTA global
 // scratch (L2 resident).  For Nv = 32 the complex work cube (256 KiB) does
 // not fit in shared memory and W and S_p live in per-CTA global scratch.
+#include <algorithm>
 #include <cstdio>
 
 #include "common.cuh"
@@ -1283,6 +1284,10 @@ __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict_
     __syncthreads();   // Qs/red reuse by the next distribution
 }
 
+}  // namespace bdgfs
+#include "vhs_tree.cuh"
+namespace bdgfs {
+
 struct KArgs {
     bdgfs_vhs_grid grids[2];
     bdgfs_vhs_batch batches[4];
@@ -1430,7 +1435,18 @@ struct Entry {
     int (*run)(const bdgfs_vhs_grid*, int, const bdgfs_vhs_batch*, int, int, void*, size_t,
                uint64_t*, cudaStream_t);
     size_t (*per)(int, size_t*);
+    int maxM;                       // largest M of the entry's code (0: any)
 };
+
+static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                       int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                       uint64_t* counter, cudaStream_t st);
+
+static size_t per_tree(int maxM, size_t* smem)
+{
+    *smem = QLayoutTree::smem_bytes(maxM);
+    return QLayoutTree::scratch_bytes();
+}
 
 #define VARIANT(T, N, NT, WG, SG) Variant<T, N, NT, WG, SG>
 #define VARIANTG(T, N, NT, GR) Variant<T, N, NT, false, false, GR>
@@ -1489,12 +1505,15 @@ static const Entry kEntries[] = {
     // the same with each thread's z-pass spectra in tensor memory
     {0, 24, 0, 320, &launch<float, 320, VariantP2<true, true, true>, NoVariant>,
      &entry_per_cta<float, 320, VariantP2<true, true, true>, NoVariant>},
+    // 24^3 by axis-wise shifts shared between directions (vhs_tree.cuh)
+    {0, 24, 0, tree::NT, &launch_tree, &per_tree, tree::kMaxM},
 };
 static constexpr int kNumEntries = int(sizeof(kEntries) / sizeof(kEntries[0]));
 
 static bool entry_matches(const Entry& e, const bdgfs_vhs_grid* grids, int ngrids)
 {
     if (e.fp64 != grids[0].fp64) return false;
+    if (e.maxM && grids[0].M > e.maxM) return false;
     if (ngrids == 1) return e.n1 == 0 && e.n0 == grids[0].Nv;
     if (e.n1 == 0) return false;
     const int a = grids[0].Nv, b = grids[1].Nv;
@@ -1557,6 +1576,56 @@ static int launch(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch
     if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), st) != cudaSuccess)
         return BDGFS_ECUDA;
     k<<<unsigned(nblk), NT, smem, st>>>(a);
+    return cuda_status(cudaGetLastError());
+}
+
+// The shift-tree kernel.  The exact-Nyquist mode (BDGFS_EXACT) has a second
+// transform per direction that does not factor; it runs on the
+// spectra-in-TMEM variant.  Scratch: tickets and slots of partial gains for
+// distributions split over radii (tree_split), as many as fit.
+static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                       int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                       uint64_t* counter, cudaStream_t st)
+{
+    if (flags & BDGFS_EXACT)
+        return launch<float, 320, VariantP2<true, true, true>, NoVariant>(
+            grids, ngrids, batches, nbatch, flags, scratch, scratch_bytes, counter, st);
+    TreeArgs a{};
+    a.g = grids[0];
+    a.nbatch = nbatch;
+    a.flags = flags;
+    a.counter = reinterpret_cast<unsigned long long*>(counter);
+    int64_t total = 0;
+    bool dev_count = false;
+    for (int b = 0; b < nbatch; ++b) {
+        a.batches[b] = batches[b];
+        total += batches[b].ndof;
+        dev_count = dev_count || batches[b].count;
+    }
+    if (total == 0) return BDGFS_OK;
+    if (scratch_bytes < QLayoutP2::scratch_bytes()) return BDGFS_ESCRATCH;
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return BDGFS_ECUDA;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return BDGFS_ECUDA;
+    const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
+    const size_t room = scratch_bytes - std::min(scratch_bytes, size_t(base - reinterpret_cast<uintptr_t>(scratch)));
+    const int64_t fit = int64_t(room / (QLayoutTree::slot_bytes() + 256));
+    if (fit < 1) return BDGFS_ESCRATCH;
+    a.tickets = reinterpret_cast<uint32_t*>(base);
+    a.slots = reinterpret_cast<unsigned char*>(base + (size_t(fit) * sizeof(uint32_t) + 255) / 256 * 256);
+    int64_t parts = std::min(a.g.Nrho, tree::kMaxSplit);
+    if (!dev_count) parts = tree_split(total, fit, a.g.Nrho, nsm);
+    if (parts > 1) {
+        a.nslots = fit;
+        if (cudaMemsetAsync(a.tickets, 0, size_t(std::min(total, fit)) * sizeof(uint32_t), st) != cudaSuccess)
+            return BDGFS_ECUDA;
+    }
+    const int64_t nblk = std::min(std::min<int64_t>(nsm, fit), total * parts);
+    const size_t smem = QLayoutTree::smem_bytes(a.g.M);
+    if (const int rc = smem_optin(reinterpret_cast<const void*>(vhs_tree_kernel), smem)) return rc;
+    if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), st) != cudaSuccess) return BDGFS_ECUDA;
+    vhs_tree_kernel<<<unsigned(nblk), tree::NT, smem, st>>>(a);
     return cuda_status(cudaGetLastError());
 }
 

@@ -1,0 +1,159 @@
+"""The shift-tree form of the 24^3 FP32 collision kernel: direction sets with
+every kind of tree node, work split over radii, ragged lists, and rows that
+are not 16-byte aligned.
+
+Reference: the FP64 oracle (<= 1e-3 of Q and 1e-5 of the loss term, the bounds
+of the other FP32 variants), and between two runs of the kernel that differ
+only in how radii are split over CTAs, 2e-5 of Q: the partial sums of the gain
+are associated differently, and Q's gain-loss cancellation turns 1e-7 of the
+terms into about 1e-5 of Q."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import mixed_maxwellians, oracle_for, rel_l2, vhs_cfg
+
+pytestmark = pytest.mark.gpu
+
+TREE = 10                               # tile index among the 24^3 FP32 variants
+
+
+def _setup(Nrho, M, ssrule=None):
+    from frfs_b200.backend import CUDABackend
+    from frfs_b200.scattering import DGFSVHSGLLScatteringModel
+    from frfs_b200.velocitymesh import DGFSVelocityMesh
+    cfg = vhs_cfg(24, Nrho, M, 6, extra=f'tile = {TREE}')
+    if ssrule:
+        cfg.set('spherical-design-rule', 'ssrule', str(ssrule))
+    be = CUDABackend(cfg)
+    vm = DGFSVelocityMesh(be, cfg)
+    return be, vm, DGFSVHSGLLScatteringModel(be, cfg, vm)
+
+
+def _rows(vm, n, seed=5):
+    rng = np.random.default_rng(seed)
+    return torch.from_numpy(np.stack([mixed_maxwellians(vm.cv(), rng) for _ in range(n)])).float().cuda()
+
+
+def _check(vm, f, q, rows):
+    orc = oracle_for(vm)
+    for i in rows:
+        F = f[i].double().cpu().numpy()
+        Qo, got = orc.Q(F), q[i].double().cpu().numpy()
+        assert rel_l2(got, Qo) < 1e-3, i
+        assert np.linalg.norm(got - Qo) < 1e-5 * np.linalg.norm(orc.gain_loss(F)[1]), i
+
+
+def _design(tmp_path, half):
+    half = np.asarray(half, float)
+    half = half / np.linalg.norm(half, axis=1, keepdims=True)
+    p = tmp_path / 'design.txt'
+    np.savetxt(p, np.concatenate([half, -half]), fmt='%.17g')
+    return p
+
+
+RNG = np.random.default_rng(0)
+DESIGNS = {
+    # no shared component: as many nodes and leaves as directions
+    'generic': RNG.normal(size=(5, 3)),
+    # one x-node; y-nodes with a mirrored leaf pair, an unmirrored one, and
+    # two leaves; opposite and repeated directions; zero components
+    'shared': [(1, .5, .7), (1, .5, -.7), (1, -.5, .7), (-1, -.5, .9 - .2), (1, .5, .7), (0, 0, 1),
+               (0, 1, 0), (0, -1, 0), (1, 0, 0), (0, .6, .8), (0, .6, -.8)],
+    'largest': RNG.normal(size=(48, 3)),
+}
+
+
+@pytest.mark.parametrize('name', list(DESIGNS))
+def test_direction_trees(cuda, tmp_path, name):
+    half = DESIGNS[name]
+    be, vm, sm = _setup(4, len(half), _design(tmp_path, half))
+    f = _rows(vm, 2)
+    q = torch.full_like(f, float('nan'))
+    sm.collide(f, q, project=False)
+    _check(vm, f, q, (0, 1))
+
+
+def test_too_many_directions_has_no_tree(cuda, tmp_path):
+    from frfs_b200.autotune import variants
+    half = np.random.default_rng(1).normal(size=(49, 3))
+    cfg_path = _design(tmp_path, half)
+    be, vm, sm48 = _setup(2, 12)
+    from frfs_b200.scattering import VHSGrid
+    sz = np.loadtxt(cfg_path)[:49]
+    g = VHSGrid(24, vm.L(), vm.qz(), vm.qw(), sz, vm.sw(), 0.38, 1.0, vm.cw(), vm.c0(), torch.float32, be.device)
+    assert len(variants([g])) == len(variants([sm48.grid])) - 1
+
+
+@pytest.mark.parametrize('M', [12, 6])
+@pytest.mark.parametrize('n', [1, 13, 75, 149, 297])
+def test_split_over_radii_agrees(cuda, M, n):
+    """Short lists cut the radii into parts (1 row: one part per radius; the
+    others fewer, or none); 600 rows are not cut."""
+    be, vm, sm = _setup(12, M)
+    f = _rows(vm, 8)[torch.arange(n) % 8].contiguous()
+    q = torch.full_like(f, float('nan'))
+    mom = torch.full((n, 10), float('nan'), dtype=torch.float64, device=f.device)
+    sm.collide(f, q, moments=mom)
+    big = f[torch.arange(600) % n].contiguous()
+    qb = torch.empty_like(big)
+    sm.collide(big, qb)
+    assert float((q - qb[:n]).double().norm() / qb[:n].double().norm()) < 2e-5
+    assert torch.isfinite(mom).all() and float(mom[:, 5:].abs().max()) < 1e-12
+    # the same launch again: bitwise (the parts are added in order)
+    q2 = torch.empty_like(q)
+    sm.collide(f, q2)
+    assert torch.equal(q, q2)
+    if n == 1:
+        sm.collide(f, q, project=False)
+        _check(vm, f, q, (0,))
+
+
+def test_device_list_and_unaligned_rows(cuda):
+    """A device index list with a device count (the split follows the count),
+    entries out of range skipped; rows at a 4-byte offset; in place."""
+    be, vm, sm = _setup(12, 12)
+    n3 = 24**3
+    f = _rows(vm, 8)[torch.arange(40) % 8].contiguous()
+    want = torch.empty_like(f)
+    sm.collide(f, want)
+    idx = torch.tensor([31, 2, 17, -1, 40, 5], dtype=torch.int32, device=f.device)
+    for count in (0, 1, 6):
+        q = torch.zeros_like(f)
+        cnt = torch.tensor([count], dtype=torch.int64, device=f.device)
+        sm.collider([(0, f, q, None)], index=idx, count=cnt)
+        done = [i for i in idx[:count].tolist() if 0 <= i < 40]
+        for i in range(40):
+            if i in done:
+                assert float((q[i] - want[i]).norm() / want[i].norm()) < 2e-5
+            else:
+                assert not bool(q[i].any())
+    g = torch.empty(3 * n3 + 1, device=f.device)[1:].view(3, n3)
+    g.copy_(f[:3])
+    q = torch.empty(3 * n3 + 1, device=f.device)[1:].view(3, n3)
+    assert g.data_ptr() % 16 == 4
+    sm.collide(g, q)
+    assert float((q - want[:3]).norm() / want[:3].norm()) < 2e-5
+    h = f[:3].clone()
+    sm.collide(h, h)
+    assert float((h - want[:3]).norm() / want[:3].norm()) < 2e-5
+
+
+def test_scratch_limits(cuda):
+    """One CTA's scratch is enough; less than a slot is refused."""
+    import ctypes as C
+    from frfs_b200 import _lib
+    be, vm, sm = _setup(12, 12)
+    f = _rows(vm, 5)
+    want, q = torch.empty_like(f), torch.full_like(f, float('nan'))
+    sm.collide(f, want)
+    arr = (_lib.VhsGrid * 1)(sm.grid.struct)
+    bs = (_lib.VhsBatch * 1)(_lib.VhsBatch(grid=0, ndof=5, f=f.data_ptr(), Q=q.data_ptr()))
+    counter = torch.zeros(1, dtype=torch.int64, device=f.device)
+    per = _lib.lib().bdgfs_vhs_scratch_bytes(arr, 1, 1)
+    s = torch.empty(per, dtype=torch.uint8, device=f.device)
+    call = lambda n: _lib.lib().bdgfs_vhs_collide(arr, 1, bs, 1, 1, s.data_ptr(), C.c_size_t(n),
+                                                  counter.data_ptr(), _lib.stream_ptr())
+    assert call(per) == 0
+    assert float((q - want).norm() / want.norm()) < 2e-5
+    assert call(1024) == -5
