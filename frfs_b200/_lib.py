@@ -20,7 +20,7 @@ EXPORTS = (
     'bdgfs_vhs_collide_static', 'bdgfs_wait_probe',
     'bdgfs_fr_disu', 'bdgfs_fr_invmass', 'bdgfs_fr_bc_update', 'bdgfs_fr_rhs', 'bdgfs_fr_rhs_gather',
     'bdgfs_fr_bc_update_gather', 'bdgfs_fr_rhs_tensor',
-    'bdgfs_moments', 'bdgfs_residual', 'bdgfs_status_check',
+    'bdgfs_moments', 'bdgfs_macroscopic', 'bdgfs_residual', 'bdgfs_status_check',
     'bdgfs_gemm', 'bdgfs_colsum', 'bdgfs_adamw', 'bdgfs_relmse',
     'bdgfs_hybrid_classify', 'bdgfs_hybrid_project', 'bdgfs_hybrid_scatter',
     'bdgfs_hybrid_project_scatter', 'bdgfs_hybrid_heads', 'bdgfs_hybrid_shift',
@@ -171,6 +171,7 @@ def lib():
             'bdgfs_fr_bc_update_gather': [vp, vp, vp, vp, vp],
             'bdgfs_fr_rhs_tensor': [vp, vp, vp, vp, vp, vp, dbl, dbl, vp, dbl, vp, dbl, vp],
             'bdgfs_moments': [vp, i64, i32, i32, vp, dbl, vp, vp],
+            'bdgfs_macroscopic': [vp, i64, i32, i32, vp, dbl, vp, vp, vp, vp, vp, vp],
             'bdgfs_residual': [vp, vp, i64, i32, vp, vp],
             'bdgfs_status_check': [vp, i64, i32, vp, vp],
             'bdgfs_gemm': [C.c_void_p, vp],

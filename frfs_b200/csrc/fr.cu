@@ -683,44 +683,6 @@ __global__ void __launch_bounds__(256) bc_update_kernel(const bdgfs_fr_eles el,
     }
 }
 
-// raw FP64 velocity moments of each distribution:
-// sum f, sum c f (3), sum c_i c_j f (6: xx xy xz yy yz zz), sum |c|^2 c f (3)
-template <typename T>
-__global__ void __launch_bounds__(256) moments_kernel(const T* __restrict__ f, int Nv,
-                                                      const double* __restrict__ c0, double cw,
-                                                      double* __restrict__ out)
-{
-    __shared__ double red[13 * 8];
-    const int64_t n = int64_t(Nv) * Nv * Nv;
-    const T* fd = f + int64_t(blockIdx.x) * n;
-    double m[13];
-#pragma unroll
-    for (int j = 0; j < 13; ++j) m[j] = 0.0;
-    for (int64_t v = threadIdx.x; v < n; v += blockDim.x) {
-        const double cx = c0[v / (int64_t(Nv) * Nv)], cy = c0[(v / Nv) % Nv], cz = c0[v % Nv];
-        const double fv = double(fd[v]);
-        const double c2 = cx * cx + cy * cy + cz * cz;
-        m[0] += fv;
-        m[1] += cx * fv; m[2] += cy * fv; m[3] += cz * fv;
-        m[4] += cx * cx * fv; m[5] += cx * cy * fv; m[6] += cx * cz * fv;
-        m[7] += cy * cy * fv; m[8] += cy * cz * fv; m[9] += cz * cz * fv;
-        m[10] += c2 * cx * fv; m[11] += c2 * cy * fv; m[12] += c2 * cz * fv;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < 13; ++j) {
-        double x = m[j];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) red[warp * 13 + j] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < 13) {
-        double s = 0.0;
-        for (int w = 0; w < int(blockDim.x >> 5); ++w) s += red[w * 13 + threadIdx.x];
-        out[int64_t(blockIdx.x) * 13 + threadIdx.x] = s * cw;
-    }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256) residual_kernel(const T* __restrict__ a,
                                                        const T* __restrict__ b, int64_t n,
@@ -1019,20 +981,6 @@ extern "C" int32_t bdgfs_fr_rhs_tensor(const bdgfs_fr_eles* el, const bdgfs_fr_w
     GO(2, 4, 8, 2) GO(2, 9, 12, 3) GO(2, 16, 16, 4) GO(3, 8, 24, 2) GO(3, 27, 54, 3)
 #undef GO
     return BDGFS_EUNSUPPORTED;
-}
-
-extern "C" int32_t bdgfs_moments(const void* f, int64_t ndof, int32_t Nv, int32_t fp64,
-                                 const double* c0, double cw, double* out, void* stream)
-{
-    if (!f || !c0 || !out || ndof < 0 || Nv < 1) return BDGFS_EINVAL;
-    if (ndof == 0) return BDGFS_OK;
-    if (ndof > 2147483647LL) return BDGFS_EINVAL;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (fp64)
-        moments_kernel<double><<<unsigned(ndof), 256, 0, st>>>(static_cast<const double*>(f), Nv, c0, cw, out);
-    else
-        moments_kernel<float><<<unsigned(ndof), 256, 0, st>>>(static_cast<const float*>(f), Nv, c0, cw, out);
-    return cuda_status(cudaGetLastError());
 }
 
 extern "C" int32_t bdgfs_residual(const void* a, const void* b, int64_t n, int32_t fp64,

@@ -497,7 +497,7 @@ class DGFSSystem:
 def raw_moments(f, vm):
     """FP64 raw moments [ndof][13] (bdgfs_moments)."""
     n3 = vm.vsize()
-    f2 = f.reshape(-1, n3)
+    f2 = f.reshape(-1, n3).contiguous()
     out = torch.empty(f2.shape[0], 13, dtype=torch.float64, device=f.device)
     c0 = torch.as_tensor(vm.c0(), dtype=torch.float64, device=f.device)
     L = _lib.lib()
@@ -509,7 +509,20 @@ def raw_moments(f, vm):
 
 def macroscopic(f, vm):
     """rho, U[3], T, q[3], P[6] per DOF from the FP64 raw moments, with the
-    definitions of frfs/plugins/dgfsmomwriterstd.py:151-213 (3-D, mr = 1)."""
+    definitions of frfs/plugins/dgfsmomwriterstd.py:151-213 (3-D, mr = 1);
+    one launch (bdgfs_macroscopic)."""
+    if vm.Nv() <= 64:
+        n3 = vm.vsize()
+        f2 = f.reshape(-1, n3).contiguous()
+        nd = f2.shape[0]
+        new = lambda *s: torch.empty(*s, dtype=torch.float64, device=f.device)
+        rho, U, T, q, P = new(nd), new(nd, 3), new(nd), new(nd, 3), new(nd, 6)
+        c0 = np.ascontiguousarray(vm.c0(), dtype=np.float64)
+        _lib.check(_lib.lib().bdgfs_macroscopic(
+            f2.data_ptr(), nd, vm.Nv(), int(f.dtype == torch.float64), c0.ctypes.data, float(vm.cw()),
+            rho.data_ptr(), U.data_ptr(), T.data_ptr(), q.data_ptr(), P.data_ptr(),
+            _lib.stream_ptr()), 'bdgfs_macroscopic')
+        return rho, U, T, q, P
     m = raw_moments(f, vm)
     rho = m[:, 0]
     U = m[:, 1:4] / rho[:, None]

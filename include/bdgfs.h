@@ -265,6 +265,16 @@ int32_t bdgfs_fr_rhs_tensor(const bdgfs_fr_eles* el, const bdgfs_fr_walls* wl,
 int32_t bdgfs_moments(const void* f, int64_t ndof, int32_t Nv, int32_t fp64,
                       const double* c0, double cw, double* out, void* stream);
 
+/* Macroscopic fields of ndof distributions from the same moments, in FP64 and
+ * one launch: rho[ndof], U[ndof][3], T[ndof], q[ndof][3], P[ndof][6] (xx xy xz
+ * yy yz zz) with the definitions of plugins/dgfsmomwriterstd.py:151-213 (3-D,
+ * unit mass).  c0_host: the cell-centre velocities in HOST memory, read before
+ * the call returns; Nv <= 64. */
+int32_t bdgfs_macroscopic(const void* f, int64_t ndof, int32_t Nv, int32_t fp64,
+                          const double* c0_host, double cw, double* rho,
+                          double* U, double* T, double* q, double* P,
+                          void* stream);
+
 /* out2[0] = sum (a-b)^2, out2[1] = sum b^2 in FP64 (residual norm of
  * plugins/dgfsresidualstd.py:34-80). */
 int32_t bdgfs_residual(const void* a, const void* b, int64_t n, int32_t fp64,
