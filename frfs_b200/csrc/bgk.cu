@@ -37,44 +37,6 @@ __device__ __forceinline__ void row_state(const double (&U)[5], double& rho, dou
     T = (U[4] - (U[1] * U[1] + U[2] * U[2] + U[3] * U[3]) / U[0]) / (1.5 * U[0]);
 }
 
-// FP64 moments {1, c, |c|^2, cx^2, cy^2, cz^2, cx cy, cy cz, cz cx} . f of a
-// row (NA = 11), followed by {|c|^2 c} (NA = 14); block-wide partial sums
-// per thread
-template <typename T, int VEC, int NA>
-__device__ __forceinline__ void row_moments_hi(const T* __restrict__ row, int n, int Nv, const double* cs,
-                                               double (&m)[NA])
-{
-    static_assert(NA == 11 || NA == 14, "11 or 14 moment rows");
-    for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
-        Chunk<T, VEC> c;
-        c.load(row + v);
-        uint32_t ix, iy, iz;
-        vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
-        const double cx = cs[ix], cy = cs[iy];
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-            const double x = double(c.v[j]), cz = cs[iz + j];
-            const double c2x = (cx * cx + cy * cy + cz * cz) * x;
-            m[0] += x;
-            m[1] += cx * x;
-            m[2] += cy * x;
-            m[3] += cz * x;
-            m[4] += c2x;
-            m[5] += cx * cx * x;
-            m[6] += cy * cy * x;
-            m[7] += cz * cz * x;
-            m[8] += cx * cy * x;
-            m[9] += cy * cz * x;
-            m[10] += cz * cx * x;
-            if constexpr (NA == 14) {
-                m[11] += cx * c2x;
-                m[12] += cy * c2x;
-                m[13] += cz * c2x;
-            }
-        }
-    }
-}
-
 // ES Gaussian of an 11-moment row: G(c) = g[0] exp(-q(c - u)), u = g[1..3],
 // q(d) = g[4] dx^2 + g[5] dy^2 + g[6] dz^2 + g[7] dx dy + g[8] dy dz + g[9] dz dx
 // (the inverse of T_ij = T/Pr delta_ij + 2 (1 - 1/Pr)(P_ij/rho - u_i u_j)).
@@ -92,7 +54,7 @@ __device__ __forceinline__ void es_params(const double* U, double Pr, double (&g
     const double det = txx * (tyy * tzz - tyz * tyz) - txy * (txy * tzz - tyz * tzx)
                        + tzx * (txy * tyz - tyy * tzx);
     const double id = 1.0 / det;
-    g[0] = rho / (pow(kPi, 1.5) * sqrt(det));
+    g[0] = rho / (kPi * sqrt(kPi) * sqrt(det));
     g[1] = ux;
     g[2] = uy;
     g[3] = uz;
@@ -110,27 +72,6 @@ __device__ __forceinline__ double es_eval(const double* g, double cx, double cy,
     const double q = g[4] * dx * dx + g[5] * dy * dy + g[6] * dz * dz + g[7] * dx * dy + g[8] * dy * dz
                      + g[9] * dz * dx;
     return g[0] * exp(-q);
-}
-
-template <typename T, int VEC, int NA>
-__global__ void __launch_bounds__(256) hi_moments_kernel(const T* __restrict__ f, int Nv, const double* c0,
-                                                         double cw, double* __restrict__ U)
-{
-    __shared__ double red[NA * 8];
-    __shared__ double cs[kMaxNv];
-    const int64_t dof = blockIdx.x;
-    const int n = Nv * Nv * Nv;
-    for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = c0[i];
-    __syncthreads();
-    double m[NA];
-#pragma unroll
-    for (int i = 0; i < NA; ++i) m[i] = 0.0;
-    row_moments_hi<T, VEC, NA>(f + dof * int64_t(n), n, Nv, cs, m);
-    block_sum<NA>(m, red);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) U[dof * NA + i] = m[i] * cw;
-    }
 }
 
 // Shakov target of a 14-moment row: S(c) = M(c) (1 + (k q . d)(2 |d|^2 / T - 5)),
@@ -215,22 +156,6 @@ __global__ void __launch_bounds__(256) esbgk_gaussian_kernel(const double* __res
 }
 
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) bgk_moments_kernel(const T* __restrict__ f, int Nv, const double* c0,
-                                                          double cw, double* __restrict__ U)
-{
-    __shared__ double red[5 * 8];
-    __shared__ double cs[kMaxNv];
-    const int64_t dof = blockIdx.x;
-    const int n = Nv * Nv * Nv;
-    for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = c0[i];
-    __syncthreads();
-    double m[5] = {0, 0, 0, 0, 0};
-    row_moments<T, VEC>(f + dof * int64_t(n), n, Nv, cs, m);
-    block_sum<5>(m, red);
-    if (threadIdx.x < 5) U[dof * 5 + threadIdx.x] = m[threadIdx.x] * cw;
-}
-
-template <typename T, int VEC>
 __global__ void __launch_bounds__(256) bgk_maxwellian_kernel(const double* __restrict__ U, int Nv,
                                                              const double* c0, T* __restrict__ M)
 {
@@ -293,187 +218,313 @@ __device__ __forceinline__ void shakov_heat(const double* u, double Pr, double (
                + (1.0 - Pr) * (-2.0 * Pu[i] + rho * v[i] * u2 - 1.5 * rho * Tt * v[i]);
 }
 
+constexpr int kRelaxWarps = 16;                        // threads per CTA: 256 or 512
+
+// Moments of up to two rows in one walk (so both rows' loads are in flight
+// together); sums of row r in ms[r] (warp 0 writes them: read after the barrier)
+template <typename T, int VEC, int NA>
+__device__ __forceinline__ void two_row_moments(const T* __restrict__ r0, const T* __restrict__ r1, int n, int Nv,
+                                                const double* cs, double cw, double (*red)[2][NA], double (*ms)[NA])
+{
+    double m0[NA], m1[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) m0[i] = m1[i] = 0.0;
+    RowWalk w(threadIdx.x * VEC, blockDim.x * VEC, uint32_t(Nv));
+#pragma unroll 2
+    for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
+        Chunk<T, VEC> a, b;
+        if (r0) a.load(r0 + v);
+        if (r1) b.load(r1 + v);
+        if (r0) chunk_moments<T, VEC, NA>(a, cs[w.ix], cs[w.iy], cs + w.iz, m0);
+        if (r1) chunk_moments<T, VEC, NA>(b, cs[w.ix], cs[w.iy], cs + w.iz, m1);
+        w.next();
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            if (r0) m0[i] += __shfl_xor_sync(0xffffffffu, m0[i], o);
+            if (r1) m1[i] += __shfl_xor_sync(0xffffffffu, m1[i], o);
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            red[warp][0][i] = m0[i];
+            red[warp][1][i] = m1[i];
+        }
+    }
+    __syncthreads();
+    if (warp == 0 && lane < NA) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            double s = 0.0;
+            for (int k = 0; k < int(blockDim.x >> 5); ++k) s += red[k][r][lane];
+            ms[r][lane] = s * cw;
+        }
+    }
+    __syncwarp();
+}
+
+// moment rows alone (the same sums, in the same order, as inside the stage kernels)
+template <typename T, int VEC, int NA>
+__global__ void __launch_bounds__(512) row_moments_kernel(const T* __restrict__ f, int Nv, const double* c0, double cw,
+                                                          double* __restrict__ U)
+{
+    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double ms[2][NA];
+    __shared__ double cs[kMaxNv];
+    const int64_t dof = blockIdx.x;
+    const int n = Nv * Nv * Nv;
+    for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = c0[i];
+    __syncthreads();
+    two_row_moments<T, VEC, NA>(f + dof * int64_t(n), nullptr, n, Nv, cs, cw, red, ms);
+    if (threadIdx.x < NA) U[dof * NA + threadIdx.x] = ms[0][threadIdx.x];
+}
+
+// temperature-dependent collision frequency of a moment row
+__device__ __forceinline__ double collision_rate(const double* u, double prefac, double omega)
+{
+    double rho, ux, uy, uz, Tt;
+    const double u5[5] = {u[0], u[1], u[2], u[3], u[4]};
+    row_state(u5, rho, ux, uy, uz, Tt);
+    return prefac * rho * pow(Tt, 1.0 - omega);
+}
+
+// Parameters of one relaxation target: u and 1/T of the separable exponentials,
+// the leading factor, and the ES tensor's or the Shakov polynomial's numbers
+struct Target {
+    double u[3], it, am, p[10];
+};
+
+template <int NA>
+__device__ __forceinline__ void target_params(const double* u, double Pr, Target& t)
+{
+    if constexpr (NA == 11) {
+        double g[10];
+        es_params(u, Pr, g);
+#pragma unroll
+        for (int i = 0; i < 10; ++i) t.p[i] = g[i];
+    } else {
+        double rho, T;
+        const double u5[5] = {u[0], u[1], u[2], u[3], u[4]};
+        row_state(u5, rho, t.u[0], t.u[1], t.u[2], T);
+        const double pt = kPi * T;
+        t.am = rho / (pt * sqrt(pt));
+        t.it = 1.0 / T;
+        if constexpr (NA == 14) {
+            double s[7];
+            shakov_params(u, Pr, s);
+#pragma unroll
+            for (int i = 0; i < 7; ++i) t.p[i] = s[i];
+        }
+    }
+}
+
+// exponential tables of the targets (NA != 11), all threads
+__device__ __forceinline__ void target_tables(const Target* t, int nt, int Nv, const double* cs,
+                                              double (*ex)[3][kMaxNv])
+{
+    for (int i = threadIdx.x; i < nt * 3 * Nv; i += blockDim.x) {
+        const int j = i / (3 * Nv), r = i - j * 3 * Nv, d = r / Nv, k = r - d * Nv;
+        const double c = cs[k] - t[j].u[d];
+        ex[j][d][k] = exp(-c * c * t[j].it);
+    }
+}
+
+template <int NA>
+__device__ __forceinline__ double target_at(const Target& t, const double (*ex)[kMaxNv], const double* cs, uint32_t ix,
+                                            uint32_t iy, uint32_t iz)
+{
+    if constexpr (NA == 11) {
+        return es_eval(t.p, cs[ix], cs[iy], cs[iz]);
+    } else {
+        const double m = t.am * ex[0][ix] * ex[1][iy] * ex[2][iz];
+        if constexpr (NA == 14) return m * shakov_factor(t.p, cs[ix], cs[iy], cs[iz]);
+        else return m;
+    }
+}
+
 // NA = 5: BGK (separable Maxwellians); NA = 11: ES-BGK (second moments
 // relaxed implicitly at nu/Pr, Gaussians evaluated per velocity); NA = 14:
 // Shakov (second moments at nu, heat flux at nu Pr, separable Maxwellians
 // times the heat-flux polynomial).
-template <typename T, int VEC, int NA>
-__global__ void __launch_bounds__(256) ars_kernel(const bdgfs_ars_args g)
+// AR > 0: the stage at compile time, so that a thread has all 2 AR rows of a
+// chunk (of two chunks for AR <= 2) in flight at once; AR = 0 reads the stage
+// from the arguments.  The moment algebra (pow, divisions) runs in one warp, a
+// lane per implicit stage, instead of in every thread.  Bound: HBM; the FP64
+// pipe and the conversions are about half of it.
+template <typename T, int VEC, int NA, int AR>
+__global__ void __launch_bounds__(512, NA == 5 && AR <= 2 ? 2 : 1) ars_kernel(const bdgfs_ars_args g)
 {
-    __shared__ double red[NA * 8];
+    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double ms[2][NA];                       // moments of f_0 and of L_{ar-1}
     __shared__ double cs[kMaxNv];
     __shared__ double ex[NA == 11 ? 1 : 4][3][kMaxNv];
-    __shared__ double gp[NA == 5 ? 1 : 4][10];
-    __shared__ double am[4], nu[4];
+    __shared__ Target tg[4];
+    __shared__ double nu[4];
     const int64_t dof = blockIdx.x;
-    const int Nv = g.Nv, ar = g.stage, flags = g.flags;
+    const int Nv = g.Nv, ar = AR > 0 ? AR : g.stage, flags = g.flags;
     const int n = Nv * Nv * Nv;
     const int64_t off = dof * int64_t(n);
     for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = g.c0[i];
     __syncthreads();
-
-    auto moments = [&](const T* row, double (&m)[NA]) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) m[i] = 0.0;
-        if constexpr (NA == 5) {
-            row_moments<T, VEC>(row, n, Nv, cs, m);
-        } else {
-            row_moments_hi<T, VEC, NA>(row, n, Nv, cs, m);
+    // ---- moments of f_0 and of the newest explicit part L_{ar-1}
+    const T* r0 = flags & BDGFS_ARS_MOM0 ? static_cast<const T*>(g.f[0]) + off : nullptr;
+    const T* r1 = flags & BDGFS_ARS_MOML ? static_cast<const T*>(g.L[ar - 1]) + off : nullptr;
+    if (r0 || r1) two_row_moments<T, VEC, NA>(r0, r1, n, Nv, cs, g.cw, red, ms);
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        if (lane < NA) {
+            if (r0) g.U[0][dof * NA + lane] = ms[0][lane];
+            if (r1) g.LU[ar - 1][dof * NA + lane] = ms[1][lane];
         }
-        block_sum<NA>(m, red);
+        __syncwarp();
+        // lane j - 1 holds moment row U_j, j = 1..ar (further lanes repeat U_ar).
+        // Stage moments: U_ar = U_0 + dt sum_j ae_j LU_j (the relaxation
+        // conserves the first five); higher moments relax implicitly
+        const int j = min(lane + 1, ar);
+        if (flags & (BDGFS_ARS_MOMU | BDGFS_ARS_DIST)) {
+            double u[NA];
 #pragma unroll
-        for (int i = 0; i < NA; ++i) m[i] *= g.cw;
-    };
-    // temperature-dependent collision frequency of a moment row
-    auto rate = [&](const double* u) {
-        double rho, ux, uy, uz, Tt;
-        double u5[5] = {u[0], u[1], u[2], u[3], u[4]};
-        row_state(u5, rho, ux, uy, uz, Tt);
-        return g.prefac * rho * pow(Tt, 1.0 - g.omega);
-    };
-
-    double U0[NA], LUl[NA], Uar[NA];
-    // ---- moments of f_0 (updateMom / moment)
-    if (flags & BDGFS_ARS_MOM0) {
-        moments(static_cast<const T*>(g.f[0]) + off, U0);
-        if (threadIdx.x == 0)
-            for (int i = 0; i < NA; ++i) g.U[0][dof * NA + i] = U0[i];
-    } else if (flags & BDGFS_ARS_MOMU) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) U0[i] = g.U[0][dof * NA + i];
-    }
-    // ---- moments of the newest explicit part L_{ar-1}
-    if (flags & BDGFS_ARS_MOML) {
-        moments(static_cast<const T*>(g.L[ar - 1]) + off, LUl);
-        if (threadIdx.x == 0)
-            for (int i = 0; i < NA; ++i) g.LU[ar - 1][dof * NA + i] = LUl[i];
-    }
-    // ---- stage moments: U_ar = U_0 + dt sum_j ae_j LU_j (the relaxation
-    // conserves the first five); higher moments relax implicitly
-    if (flags & BDGFS_ARS_MOMU) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) {
-            double s = U0[i];
-            for (int j = 0; j < ar; ++j) {
-                const double lu = (j == ar - 1 && (flags & BDGFS_ARS_MOML)) ? LUl[i] : g.LU[j][dof * NA + i];
-                s += g.dt * g.ae[j] * lu;
-            }
-            Uar[i] = s;
-        }
-        if constexpr (NA >= 11) {
-            // second moments: rate nu/Pr (ES-BGK) or nu (Shakov) towards the Maxwellian's
-            const double s2 = NA == 11 ? 1.0 / g.Pr : 1.0;
-            double num[6];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) num[k] = Uar[5 + k];
-            for (int j = 1; j < ar; ++j) {
-                const double* uj = g.U[j] + dof * NA;
-                double t[6];
-                maxwell_second(uj, t);
-                const double w = g.ai[j - 1] * g.dt * rate(uj) * s2;
-#pragma unroll
-                for (int k = 0; k < 6; ++k) num[k] += w * (t[k] - uj[5 + k]);
-            }
-            double t[6];
-            maxwell_second(Uar, t);
-            const double w = g.ai[ar - 1] * g.dt * rate(Uar) * s2;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) Uar[5 + k] = (num[k] + w * t[k]) / (1.0 + w);
-        }
-        if constexpr (NA == 14) {
-            // heat flux: dQ/dt = nu (Q(M) + (1 - Pr)(q - Q) - Pr Q), -Pr Q implicit
-            double num[3] = {Uar[11], Uar[12], Uar[13]};
-            for (int j = 1; j < ar; ++j) {
-                const double* uj = g.U[j] + dof * NA;
-                double h[3];
-                shakov_heat(uj, g.Pr, h);
-                const double w = g.ai[j - 1] * g.dt * rate(uj);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) num[k] += w * (h[k] - g.Pr * uj[11 + k]);
-            }
-            double h[3];
-            shakov_heat(Uar, g.Pr, h);
-            const double w = g.ai[ar - 1] * g.dt * rate(Uar);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) Uar[11 + k] = (num[k] + w * h[k]) / (1.0 + g.Pr * w);
-        }
-        if (threadIdx.x == 0)
-            for (int i = 0; i < NA; ++i) g.U[ar][dof * NA + i] = Uar[i];
-    }
-    if (!(flags & BDGFS_ARS_DIST)) return;
-
-    // ---- relaxation targets of U_1..U_ar (Maxwellians, ES Gaussians or
-    // Shakov distributions) and their collision frequencies
-    for (int j = 1; j <= ar; ++j) {
-        double u[NA];
-#pragma unroll
-        for (int i = 0; i < NA; ++i) u[i] = (j == ar && (flags & BDGFS_ARS_MOMU)) ? Uar[i] : g.U[j][dof * NA + i];
-        if (threadIdx.x == 0) nu[j - 1] = rate(u);
-        if constexpr (NA == 11) {
-            if (threadIdx.x == 0) {
-                double gj[10];
-                es_params(u, g.Pr, gj);
-#pragma unroll
-                for (int i = 0; i < 10; ++i) gp[j - 1][i] = gj[i];
-            }
-        } else {
-            double rho, ux, uy, uz, Tt;
-            double u5[5] = {u[0], u[1], u[2], u[3], u[4]};
-            row_state(u5, rho, ux, uy, uz, Tt);
-            if (threadIdx.x == 0) am[j - 1] = rho / pow(kPi * Tt, 1.5);
-            const double it = 1.0 / Tt;
-            for (int i = threadIdx.x; i < 3 * Nv; i += blockDim.x) {
-                const int d = i / Nv, k = i - d * Nv;
-                const double c = cs[k] - (d == 0 ? ux : d == 1 ? uy : uz);
-                ex[j - 1][d][k] = exp(-c * c * it);
-            }
-            if constexpr (NA == 14) {
-                if (threadIdx.x == 0) {
-                    double sj[7];
-                    shakov_params(u, g.Pr, sj);
-#pragma unroll
-                    for (int i = 0; i < 7; ++i) gp[j - 1][i] = sj[i];
+            for (int i = 0; i < NA; ++i) {
+                if (j < ar || !(flags & BDGFS_ARS_MOMU)) {
+                    // U_j of the implicit parts: needed for the target, and for
+                    // the higher moments' history
+                    u[i] = (flags & BDGFS_ARS_DIST) || NA > 5 || j == ar ? g.U[j][dof * NA + i] : 0.0;
+                } else {
+                    double s = r0 ? ms[0][i] : g.U[0][dof * NA + i];
+                    for (int k = 0; k < ar; ++k)
+                        s += g.dt * g.ae[k] * (k == ar - 1 && r1 ? ms[1][i] : g.LU[k][dof * NA + i]);
+                    u[i] = s;
                 }
             }
+            double rate = 0.0;
+            if (NA > 5 || (flags & BDGFS_ARS_DIST)) rate = collision_rate(u, g.prefac, g.omega);
+            if constexpr (NA >= 11) {
+                if (flags & BDGFS_ARS_MOMU) {
+                    // second moments: rate nu/Pr (ES-BGK) or nu (Shakov) towards the Maxwellian's
+                    const double w = g.ai[j - 1] * g.dt * rate, w2 = NA == 11 ? w / g.Pr : w;
+                    double t[6];
+                    maxwell_second(u, t);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        const double part = w2 * (t[k] - u[5 + k]);
+                        double num = u[5 + k];
+                        for (int q = 1; q < ar; ++q) num += __shfl_sync(0xffffffffu, part, q - 1);
+                        if (j == ar) u[5 + k] = (num + w2 * t[k]) / (1.0 + w2);
+                    }
+                    if constexpr (NA == 14) {
+                        // heat flux: dQ/dt = nu (Q(M) + (1 - Pr)(q - Q) - Pr Q), -Pr Q implicit
+                        double h[3];
+                        shakov_heat(u, g.Pr, h);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            const double part = w * (h[k] - g.Pr * u[11 + k]);
+                            double num = u[11 + k];
+                            for (int q = 1; q < ar; ++q) num += __shfl_sync(0xffffffffu, part, q - 1);
+                            if (j == ar) u[11 + k] = (num + w * h[k]) / (1.0 + g.Pr * w);
+                        }
+                    }
+                }
+            }
+            if (lane == ar - 1 && (flags & BDGFS_ARS_MOMU)) {
+#pragma unroll
+                for (int i = 0; i < NA; ++i) g.U[ar][dof * NA + i] = u[i];
+            }
+            if (lane < ar && (flags & BDGFS_ARS_DIST)) {
+                nu[lane] = rate;
+                target_params<NA>(u, g.Pr, tg[lane]);
+            }
         }
     }
+    if (!(flags & BDGFS_ARS_DIST)) return;
     __syncthreads();
-    auto target = [&](int j, uint32_t ix, uint32_t iy, uint32_t izq) -> double {
-        if constexpr (NA == 11) {
-            return es_eval(gp[j], cs[ix], cs[iy], cs[izq]);
-        } else {
-            const double m = am[j] * ex[j][0][ix] * ex[j][1][iy] * ex[j][2][izq];
-            if constexpr (NA == 14) return m * shakov_factor(gp[j], cs[ix], cs[iy], cs[izq]);
-            else return m;
-        }
-    };
+    if constexpr (NA != 11) {
+        target_tables(tg, ar, Nv, cs, ex);
+        __syncthreads();
+    }
+
     const double dt = g.dt;
     const double aii = g.ai[ar - 1] * dt * nu[ar - 1];
     const double inv = 1.0 / (1.0 + aii);
-    for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
-        uint32_t ix, iy, iz;
-        vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
-        double acc[VEC];
-        Chunk<T, VEC> c;
-        c.load(static_cast<const T*>(g.f[0]) + off + v);
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) acc[q] = double(c.v[q]);
-        for (int j = 0; j < ar; ++j) {
-            c.load(static_cast<const T*>(g.L[j]) + off + v);
-            const double w = g.ae[j] * dt;
-#pragma unroll
-            for (int q = 0; q < VEC; ++q) acc[q] += w * double(c.v[q]);
-        }
-        for (int j = 1; j < ar; ++j) {
-            c.load(static_cast<const T*>(g.f[j]) + off + v);
-            const double w = g.ai[j - 1] * dt * nu[j - 1];
-#pragma unroll
-            for (int q = 0; q < VEC; ++q) acc[q] += w * (target(j - 1, ix, iy, iz + q) - double(c.v[q]));
-        }
+    const T* f0 = static_cast<const T*>(g.f[0]) + off;
+    T* fout = static_cast<T*>(g.fout) + off;
+    auto finish = [&](int v, const RowWalk& w, double (&acc)[VEC]) {
         Chunk<T, VEC> o;
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) o.v[q] = T((acc[q] + aii * target(ar - 1, ix, iy, iz + q)) * inv);
-        o.store(static_cast<T*>(g.fout) + off + v);
+        for (int q = 0; q < VEC; ++q)
+            o.v[q] = T((acc[q] + aii * target_at<NA>(tg[ar - 1], ex[NA == 11 ? 0 : ar - 1], cs, w.ix, w.iy, w.iz + q)) * inv);
+        o.store(fout + v);
+    };
+    auto add_l = [&](int j, const Chunk<T, VEC>& c, double (&acc)[VEC]) {
+        const double w = g.ae[j] * dt;
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) acc[q] += w * double(c.v[q]);
+    };
+    auto add_f = [&](int j, const Chunk<T, VEC>& c, const RowWalk& x, double (&acc)[VEC]) {
+        const double w = g.ai[j - 1] * dt * nu[j - 1];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q)
+            acc[q] += w * (target_at<NA>(tg[j - 1], ex[NA == 11 ? 0 : j - 1], cs, x.ix, x.iy, x.iz + q) - double(c.v[q]));
+    };
+    RowWalk w(threadIdx.x * VEC, blockDim.x * VEC, uint32_t(Nv));
+    if constexpr (AR > 0) {
+        const T* L[AR];
+        const T* F[AR];
+#pragma unroll
+        for (int j = 0; j < AR; ++j) {
+            L[j] = static_cast<const T*>(g.L[j]) + off;
+            F[j] = j ? static_cast<const T*>(g.f[j]) + off : f0;
+        }
+        auto step = [&](int v, const Chunk<T, VEC> (&cf)[AR], const Chunk<T, VEC> (&cl)[AR]) {
+            double acc[VEC];
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) acc[q] = double(cf[0].v[q]);
+#pragma unroll
+            for (int j = 0; j < AR; ++j) add_l(j, cl[j], acc);
+#pragma unroll
+            for (int j = 1; j < AR; ++j) add_f(j, cf[j], w, acc);
+            finish(v, w, acc);
+            w.next();
+        };
+        constexpr int U = AR <= 2 ? 2 : 1;             // chunks in flight
+        const int st = int(blockDim.x) * VEC;
+        for (int v = threadIdx.x * VEC; v < n; v += U * st) {
+            Chunk<T, VEC> cf[U][AR], cl[U][AR];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                if (v + k * st < n) {
+#pragma unroll
+                    for (int j = 0; j < AR; ++j) {
+                        cf[k][j].load(F[j] + v + k * st);
+                        cl[k][j].load(L[j] + v + k * st);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (v + k * st < n) step(v + k * st, cf[k], cl[k]);
+        }
+    } else {
+        for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
+            double acc[VEC];
+            Chunk<T, VEC> c;
+            c.load(f0 + v);
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) acc[q] = double(c.v[q]);
+            for (int j = 0; j < ar; ++j) {
+                c.load(static_cast<const T*>(g.L[j]) + off + v);
+                add_l(j, c, acc);
+            }
+            for (int j = 1; j < ar; ++j) {
+                c.load(static_cast<const T*>(g.f[j]) + off + v);
+                add_f(j, c, w, acc);
+            }
+            finish(v, w, acc);
+            w.next();
+        }
     }
 }
 
@@ -484,148 +535,129 @@ __global__ void __launch_bounds__(256) ars_kernel(const bdgfs_ars_args g)
 //        the heat flux with denominator a_q + Pr b dt nu)
 //   f  = (N_f + b dt nu M[U]) / (a_q + b dt nu).
 // One CTA per distribution; the newest moment rows (of f_{q-1} and of
-// L_{q-1}) are reduced in the same launch when BDGFS_BDF_MOMN is set.
-template <typename T, int VEC, int NA>
-__global__ void __launch_bounds__(256) bdf_kernel(const bdgfs_bdf_args g)
+// L_{q-1}) are reduced in the same launch when BDGFS_BDF_MOMN is set.  BQ > 0:
+// the order q at compile time (all 2 q rows of a chunk in flight); BQ = 0 reads
+// it from the arguments.  Moment algebra in one thread.  315 rows of 24^3 FP32,
+// Shakov, BDF-2: 86 -> 53 us on one B200 (512 threads a row).
+template <typename T, int VEC, int NA, int BQ>
+__global__ void __launch_bounds__(512, NA == 5 ? 2 : 1) bdf_kernel(const bdgfs_bdf_args g)
 {
-    __shared__ double red[NA * 8];
+    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double ms[2][NA];                       // moments of f_{q-1} and of L_{q-1}
     __shared__ double cs[kMaxNv];
-    __shared__ double ex[3][kMaxNv];
-    __shared__ double gp[10];
-    __shared__ double am, nu;
+    __shared__ double ex[1][3][kMaxNv];
+    __shared__ Target tg;
+    __shared__ double nu;
     const int64_t dof = blockIdx.x;
-    const int Nv = g.Nv, q = g.q, flags = g.flags;
+    const int Nv = g.Nv, q = BQ > 0 ? BQ : g.q, flags = g.flags;
     const int n = Nv * Nv * Nv;
     const int64_t off = dof * int64_t(n);
     for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = g.c0[i];
     __syncthreads();
-
-    auto moments = [&](const T* row, double (&m)[NA]) {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) m[i] = 0.0;
-        if constexpr (NA == 5) {
-            row_moments<T, VEC>(row, n, Nv, cs, m);
-        } else {
-            row_moments_hi<T, VEC, NA>(row, n, Nv, cs, m);
-        }
-        block_sum<NA>(m, red);
-#pragma unroll
-        for (int i = 0; i < NA; ++i) m[i] *= g.cw;
-    };
-    auto rate = [&](const double* u) {
-        double rho, ux, uy, uz, Tt;
-        double u5[5] = {u[0], u[1], u[2], u[3], u[4]};
-        row_state(u5, rho, ux, uy, uz, Tt);
-        return g.prefac * rho * pow(Tt, 1.0 - g.omega);
-    };
-
-    double Un[NA], LUn[NA], U[NA];
-    if (flags & BDGFS_BDF_MOMN) {
-        moments(static_cast<const T*>(g.f[q - 1]) + off, Un);
-        moments(static_cast<const T*>(g.L[q - 1]) + off, LUn);
-        if (threadIdx.x == 0)
-            for (int i = 0; i < NA; ++i) {
-                g.U[q - 1][dof * NA + i] = Un[i];
-                g.LU[q - 1][dof * NA + i] = LUn[i];
-            }
-    }
+    const bool momn = flags & BDGFS_BDF_MOMN;
+    if (momn)
+        two_row_moments<T, VEC, NA>(static_cast<const T*>(g.f[q - 1]) + off, static_cast<const T*>(g.L[q - 1]) + off, n,
+                                    Nv, cs, g.cw, red, ms);
     const double aq = g.a[q];
-    if (flags & BDGFS_BDF_MOMU) {
-        double N[NA];
-#pragma unroll
-        for (int k = 0; k < NA; ++k) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        if (momn && lane < NA) {
+            g.U[q - 1][dof * NA + lane] = ms[0][lane];
+            g.LU[q - 1][dof * NA + lane] = ms[1][lane];
+        }
+        __syncwarp();
+        if (flags & (BDGFS_BDF_MOMU | BDGFS_BDF_DIST)) {
+            // lane k forms N_k (or reads U_k), then lane 0 has the row
+            double u[NA];
+            const int k = min(lane, NA - 1);
             double s = 0.0;
-            for (int i = 0; i < q; ++i) {
-                const bool fresh = i == q - 1 && (flags & BDGFS_BDF_MOMN);
-                const double ui = fresh ? Un[k] : g.U[i][dof * NA + k];
-                const double li = fresh ? LUn[k] : g.LU[i][dof * NA + k];
-                s -= g.a[i] * ui + g.g[i] * g.dt * li;
+            if (flags & BDGFS_BDF_MOMU) {
+                for (int i = 0; i < q; ++i) {
+                    const bool fresh = i == q - 1 && momn;
+                    const double ui = fresh ? ms[0][k] : g.U[i][dof * NA + k];
+                    const double li = fresh ? ms[1][k] : g.LU[i][dof * NA + k];
+                    s -= g.a[i] * ui + g.g[i] * g.dt * li;
+                }
+            } else {
+                s = g.Unew[dof * NA + k];
             }
-            N[k] = s;
+#pragma unroll
+            for (int i = 0; i < NA; ++i) u[i] = __shfl_sync(0xffffffffu, s, i);
+            if (lane == 0) {
+                if (flags & BDGFS_BDF_MOMU) {
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) u[i] = u[i] / aq;
+                }
+                double rate = 0.0;
+                if (NA > 5 || (flags & BDGFS_BDF_DIST)) rate = collision_rate(u, g.prefac, g.omega);
+                if (flags & BDGFS_BDF_MOMU) {
+                    if constexpr (NA >= 11) {
+                        const double w = g.b * g.dt * rate * (NA == 11 ? 1.0 / g.Pr : 1.0);
+                        double t[6];
+                        maxwell_second(u, t);
+#pragma unroll
+                        for (int i = 0; i < 6; ++i) u[5 + i] = (u[5 + i] + w * t[i]) / (aq + w);
+                    }
+                    if constexpr (NA == 14) {
+                        const double w = g.b * g.dt * rate;
+                        double h[3];
+                        shakov_heat(u, g.Pr, h);
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) u[11 + i] = (u[11 + i] + w * h[i]) / (aq + g.Pr * w);
+                    }
+#pragma unroll
+                    for (int i = 0; i < NA; ++i) g.Unew[dof * NA + i] = u[i];
+                }
+                if (flags & BDGFS_BDF_DIST) {
+                    nu = rate;
+                    target_params<NA>(u, g.Pr, tg);
+                }
+            }
         }
-#pragma unroll
-        for (int k = 0; k < 5; ++k) U[k] = N[k] / aq;
-        if constexpr (NA >= 11) {
-            const double w = g.b * g.dt * rate(U) * (NA == 11 ? 1.0 / g.Pr : 1.0);
-            double t[6];
-            maxwell_second(U, t);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) U[5 + k] = (N[5 + k] + w * t[k]) / (aq + w);
-        }
-        if constexpr (NA == 14) {
-            const double w = g.b * g.dt * rate(U);
-            double h[3];
-            shakov_heat(U, g.Pr, h);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) U[11 + k] = (N[11 + k] + w * h[k]) / (aq + g.Pr * w);
-        }
-        if (threadIdx.x == 0)
-            for (int i = 0; i < NA; ++i) g.Unew[dof * NA + i] = U[i];
-    } else {
-#pragma unroll
-        for (int i = 0; i < NA; ++i) U[i] = g.Unew[dof * NA + i];
     }
     if (!(flags & BDGFS_BDF_DIST)) return;
-
-    // relaxation target of U and its collision frequency
-    if (threadIdx.x == 0) nu = rate(U);
-    if constexpr (NA == 11) {
-        if (threadIdx.x == 0) {
-            double gj[10];
-            es_params(U, g.Pr, gj);
-#pragma unroll
-            for (int i = 0; i < 10; ++i) gp[i] = gj[i];
-        }
-    } else {
-        double rho, ux, uy, uz, Tt;
-        double u5[5] = {U[0], U[1], U[2], U[3], U[4]};
-        row_state(u5, rho, ux, uy, uz, Tt);
-        if (threadIdx.x == 0) am = rho / pow(kPi * Tt, 1.5);
-        const double it = 1.0 / Tt;
-        for (int i = threadIdx.x; i < 3 * Nv; i += blockDim.x) {
-            const int d = i / Nv, k = i - d * Nv;
-            const double c = cs[k] - (d == 0 ? ux : d == 1 ? uy : uz);
-            ex[d][k] = exp(-c * c * it);
-        }
-        if constexpr (NA == 14) {
-            if (threadIdx.x == 0) {
-                double sj[7];
-                shakov_params(U, g.Pr, sj);
-#pragma unroll
-                for (int i = 0; i < 7; ++i) gp[i] = sj[i];
-            }
-        }
-    }
     __syncthreads();
-    auto target = [&](uint32_t ix, uint32_t iy, uint32_t izq) -> double {
-        if constexpr (NA == 11) {
-            return es_eval(gp, cs[ix], cs[iy], cs[izq]);
-        } else {
-            const double m = am * ex[0][ix] * ex[1][iy] * ex[2][izq];
-            if constexpr (NA == 14) return m * shakov_factor(gp, cs[ix], cs[iy], cs[izq]);
-            else return m;
-        }
-    };
+    if constexpr (NA != 11) {
+        target_tables(&tg, 1, Nv, cs, ex);
+        __syncthreads();
+    }
     const double bdn = g.b * g.dt * nu;
     const double inv = 1.0 / (aq + bdn);
+    T* fout = static_cast<T*>(g.fout) + off;
+    RowWalk w(threadIdx.x * VEC, blockDim.x * VEC, uint32_t(Nv));
+    constexpr int QB = BQ > 0 ? BQ : 1;
     for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
-        uint32_t ix, iy, iz;
-        vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
         double acc[VEC];
 #pragma unroll
         for (int j = 0; j < VEC; ++j) acc[j] = 0.0;
-        for (int i = 0; i < q; ++i) {
-            Chunk<T, VEC> cf, cl;
-            cf.load(static_cast<const T*>(g.f[i]) + off + v);
-            cl.load(static_cast<const T*>(g.L[i]) + off + v);
+        auto add = [&](int i, const Chunk<T, VEC>& cf, const Chunk<T, VEC>& cl) {
             const double wa = g.a[i], wg = g.g[i] * g.dt;
 #pragma unroll
             for (int j = 0; j < VEC; ++j) acc[j] -= wa * double(cf.v[j]) + wg * double(cl.v[j]);
+        };
+        if constexpr (BQ > 0) {
+            Chunk<T, VEC> cf[QB], cl[QB];
+#pragma unroll
+            for (int i = 0; i < QB; ++i) {
+                cf[i].load(static_cast<const T*>(g.f[i]) + off + v);
+                cl[i].load(static_cast<const T*>(g.L[i]) + off + v);
+            }
+#pragma unroll
+            for (int i = 0; i < QB; ++i) add(i, cf[i], cl[i]);
+        } else {
+            for (int i = 0; i < q; ++i) {
+                Chunk<T, VEC> cf, cl;
+                cf.load(static_cast<const T*>(g.f[i]) + off + v);
+                cl.load(static_cast<const T*>(g.L[i]) + off + v);
+                add(i, cf, cl);
+            }
         }
         Chunk<T, VEC> o;
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) o.v[j] = T((acc[j] + bdn * target(ix, iy, iz + j)) * inv);
-        o.store(static_cast<T*>(g.fout) + off + v);
+        for (int j = 0; j < VEC; ++j)
+            o.v[j] = T((acc[j] + bdn * target_at<NA>(tg, ex[0], cs, w.ix, w.iy, w.iz + j)) * inv);
+        o.store(fout + v);
+        w.next();
     }
 }
 
@@ -647,6 +679,56 @@ int32_t launch_rows(bool v4, K4 k4, K1 k1, int64_t ndof, cudaStream_t st, Args..
     return cuda_status(cudaGetLastError());
 }
 
+// Relaxation kernels: 512 threads per row when the rows are too few to fill
+// the SMs with 256 (fewer than four CTAs each), else 256
+unsigned relax_threads(int64_t ndof) { return ndof < 148 * 4 ? 512 : 256; }
+
+template <typename K, typename A>
+int32_t launch_relax(K k, const A& a, cudaStream_t st)
+{
+    k<<<unsigned(a.ndof), relax_threads(a.ndof), 0, st>>>(a);
+    return cuda_status(cudaGetLastError());
+}
+
+template <int NA>
+int32_t launch_moments(const void* f, int64_t ndof, int Nv, int fp64, const double* c0, double cw, double* U,
+                       cudaStream_t st)
+{
+    const bool v4 = Nv % 4 == 0 && a16(f);
+    const unsigned nt = relax_threads(ndof);
+#define GO(T, V) row_moments_kernel<T, V, NA><<<unsigned(ndof), nt, 0, st>>>(static_cast<const T*>(f), Nv, c0, cw, U)
+    if (fp64) {
+        if (v4) GO(double, 4);
+        else GO(double, 1);
+    } else {
+        if (v4) GO(float, 4);
+        else GO(float, 1);
+    }
+#undef GO
+    return cuda_status(cudaGetLastError());
+}
+
+template <typename T, int NA>
+int32_t launch_ars(bool v4, const bdgfs_ars_args& a, cudaStream_t st)
+{
+    if (v4) {
+        if (a.stage == 1) return launch_relax(ars_kernel<T, 4, NA, 1>, a, st);
+        if (a.stage == 2) return launch_relax(ars_kernel<T, 4, NA, 2>, a, st);
+        if (a.stage == 3) return launch_relax(ars_kernel<T, 4, NA, 3>, a, st);
+        return launch_relax(ars_kernel<T, 4, NA, 4>, a, st);
+    }
+    return launch_relax(ars_kernel<T, 1, NA, 0>, a, st);
+}
+
+template <typename T, int NA>
+int32_t launch_bdf(bool v4, const bdgfs_bdf_args& a, cudaStream_t st)
+{
+    if (v4 && a.q == 2) return launch_relax(bdf_kernel<T, 4, NA, 2>, a, st);
+    if (v4 && a.q == 3) return launch_relax(bdf_kernel<T, 4, NA, 3>, a, st);
+    if (v4) return launch_relax(bdf_kernel<T, 4, NA, 0>, a, st);
+    return launch_relax(bdf_kernel<T, 1, NA, 0>, a, st);
+}
+
 }  // namespace
 
 extern "C" int32_t bdgfs_bgk_moments(const void* f, int64_t ndof, int32_t Nv, int32_t fp64, const double* c0,
@@ -654,13 +736,7 @@ extern "C" int32_t bdgfs_bgk_moments(const void* f, int64_t ndof, int32_t Nv, in
 {
     if (!f || !c0 || !U || ndof < 0 || ndof > 2147483647LL || Nv < 1 || Nv > kMaxNv) return BDGFS_EINVAL;
     if (ndof == 0) return BDGFS_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool v4 = Nv % 4 == 0 && a16(f);
-    if (fp64)
-        return launch_rows(v4, bgk_moments_kernel<double, 4>, bgk_moments_kernel<double, 1>, ndof, st,
-                           static_cast<const double*>(f), int(Nv), c0, cw, U);
-    return launch_rows(v4, bgk_moments_kernel<float, 4>, bgk_moments_kernel<float, 1>, ndof, st,
-                       static_cast<const float*>(f), int(Nv), c0, cw, U);
+    return launch_moments<5>(f, ndof, Nv, fp64, c0, cw, U, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t bdgfs_bgk_maxwellian(const double* U, int64_t ndof, int32_t Nv, int32_t fp64,
@@ -705,16 +781,11 @@ extern "C" int32_t bdgfs_ars_stage(const bdgfs_ars_args* a, void* stream)
     }
     if (a->ndof == 0) return BDGFS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a->model == BDGFS_ARS_SHAKOV) {
-        if (a->fp64) return launch_rows(v4, ars_kernel<double, 4, 14>, ars_kernel<double, 1, 14>, a->ndof, st, *a);
-        return launch_rows(v4, ars_kernel<float, 4, 14>, ars_kernel<float, 1, 14>, a->ndof, st, *a);
-    }
-    if (a->model == BDGFS_ARS_ESBGK) {
-        if (a->fp64) return launch_rows(v4, ars_kernel<double, 4, 11>, ars_kernel<double, 1, 11>, a->ndof, st, *a);
-        return launch_rows(v4, ars_kernel<float, 4, 11>, ars_kernel<float, 1, 11>, a->ndof, st, *a);
-    }
-    if (a->fp64) return launch_rows(v4, ars_kernel<double, 4, 5>, ars_kernel<double, 1, 5>, a->ndof, st, *a);
-    return launch_rows(v4, ars_kernel<float, 4, 5>, ars_kernel<float, 1, 5>, a->ndof, st, *a);
+#define ARS_GO(NA) return a->fp64 ? launch_ars<double, NA>(v4, *a, st) : launch_ars<float, NA>(v4, *a, st);
+    if (a->model == BDGFS_ARS_SHAKOV) { ARS_GO(14) }
+    if (a->model == BDGFS_ARS_ESBGK) { ARS_GO(11) }
+    ARS_GO(5)
+#undef ARS_GO
 }
 
 extern "C" int32_t bdgfs_esbgk_moments(const void* f, int64_t ndof, int32_t Nv, int32_t fp64,
@@ -722,13 +793,7 @@ extern "C" int32_t bdgfs_esbgk_moments(const void* f, int64_t ndof, int32_t Nv, 
 {
     if (!f || !c0 || !U || ndof < 0 || ndof > 2147483647LL || Nv < 1 || Nv > kMaxNv) return BDGFS_EINVAL;
     if (ndof == 0) return BDGFS_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool v4 = Nv % 4 == 0 && a16(f);
-    if (fp64)
-        return launch_rows(v4, hi_moments_kernel<double, 4, 11>, hi_moments_kernel<double, 1, 11>, ndof, st,
-                           static_cast<const double*>(f), int(Nv), c0, cw, U);
-    return launch_rows(v4, hi_moments_kernel<float, 4, 11>, hi_moments_kernel<float, 1, 11>, ndof, st,
-                       static_cast<const float*>(f), int(Nv), c0, cw, U);
+    return launch_moments<11>(f, ndof, Nv, fp64, c0, cw, U, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t bdgfs_esbgk_gaussian(const double* U, int64_t ndof, int32_t Nv, int32_t fp64,
@@ -751,13 +816,7 @@ extern "C" int32_t bdgfs_shakov_moments(const void* f, int64_t ndof, int32_t Nv,
 {
     if (!f || !c0 || !U || ndof < 0 || ndof > 2147483647LL || Nv < 1 || Nv > kMaxNv) return BDGFS_EINVAL;
     if (ndof == 0) return BDGFS_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool v4 = Nv % 4 == 0 && a16(f);
-    if (fp64)
-        return launch_rows(v4, hi_moments_kernel<double, 4, 14>, hi_moments_kernel<double, 1, 14>, ndof, st,
-                           static_cast<const double*>(f), int(Nv), c0, cw, U);
-    return launch_rows(v4, hi_moments_kernel<float, 4, 14>, hi_moments_kernel<float, 1, 14>, ndof, st,
-                       static_cast<const float*>(f), int(Nv), c0, cw, U);
+    return launch_moments<14>(f, ndof, Nv, fp64, c0, cw, U, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t bdgfs_shakov_target(const double* U, int64_t ndof, int32_t Nv, int32_t fp64,
@@ -803,9 +862,7 @@ extern "C" int32_t bdgfs_bdf_step(const bdgfs_bdf_args* a, void* stream)
     }
     if (a->ndof == 0) return BDGFS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define BDF_GO(NA)                                                                                         \
-    return a->fp64 ? launch_rows(v4, bdf_kernel<double, 4, NA>, bdf_kernel<double, 1, NA>, a->ndof, st, *a) \
-                   : launch_rows(v4, bdf_kernel<float, 4, NA>, bdf_kernel<float, 1, NA>, a->ndof, st, *a);
+#define BDF_GO(NA) return a->fp64 ? launch_bdf<double, NA>(v4, *a, st) : launch_bdf<float, NA>(v4, *a, st);
     if (a->model == BDGFS_ARS_SHAKOV) { BDF_GO(14) }
     if (a->model == BDGFS_ARS_ESBGK) { BDF_GO(11) }
     BDF_GO(5)

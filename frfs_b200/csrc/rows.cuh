@@ -50,6 +50,74 @@ struct Chunk {
     }
 };
 
+// Walk of a row in steps of a fixed number of values: the index split kept by
+// carries instead of two divisions per step.  step < Nv^3.
+struct RowWalk {
+    uint32_t ix, iy, iz, dx, dy, dz, N;
+    __device__ __forceinline__ RowWalk(uint32_t v, uint32_t step, uint32_t Nv) : N(Nv)
+    {
+        vsplit(v, Nv, ix, iy, iz);
+        vsplit(step, Nv, dx, dy, dz);
+    }
+    __device__ __forceinline__ void next()
+    {
+        iz += dz;
+        iy += dy;
+        ix += dx;
+        if (iz >= N) { iz -= N; ++iy; }
+        if (iy >= N) { iy -= N; ++ix; }
+    }
+};
+
+// FP64 moments of a chunk added to m: {1, c, |c|^2} (NA = 5), then {cx^2, cy^2,
+// cz^2, cx cy, cy cz, cz cx} (NA = 11), then {|c|^2 c} (NA = 14).  The chunk's
+// z-sums (of x, cz x, cz^2 x, cz^3 x) come first, so a value costs one
+// conversion and 3 or 4 FP64 operations and the rest is per chunk.
+template <typename T, int VEC, int NA>
+__device__ __forceinline__ void chunk_moments(const Chunk<T, VEC>& c, double cx, double cy, const double* cz,
+                                              double (&m)[NA])
+{
+    static_assert(NA == 5 || NA == 11 || NA == 14, "5, 11 or 14 moment rows");
+    // every rounding written out: kernels that reduce the same row in the same
+    // order get the same bits, however the compiler contracts
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+        const double z = cz[j];
+        double t = double(c.v[j]);
+        s0 = __dadd_rn(s0, t);
+        t = __dmul_rn(t, z);
+        s1 = __dadd_rn(s1, t);
+        if constexpr (NA == 14) {
+            t = __dmul_rn(t, z);
+            s2 = __dadd_rn(s2, t);
+            s3 = fma(t, z, s3);
+        } else {
+            s2 = fma(t, z, s2);
+        }
+    }
+    const double a = __dmul_rn(cx, s0), b = __dmul_rn(cy, s0), r2 = fma(cx, cx, __dmul_rn(cy, cy));
+    const double e = fma(r2, s0, s2);
+    m[0] = __dadd_rn(m[0], s0);
+    m[1] = __dadd_rn(m[1], a);
+    m[2] = __dadd_rn(m[2], b);
+    m[3] = __dadd_rn(m[3], s1);
+    m[4] = __dadd_rn(m[4], e);
+    if constexpr (NA >= 11) {
+        m[5] = fma(cx, a, m[5]);
+        m[6] = fma(cy, b, m[6]);
+        m[7] = __dadd_rn(m[7], s2);
+        m[8] = fma(cx, b, m[8]);
+        m[9] = fma(cy, s1, m[9]);
+        m[10] = fma(cx, s1, m[10]);
+    }
+    if constexpr (NA == 14) {
+        m[11] = fma(cx, e, m[11]);
+        m[12] = fma(cy, e, m[12]);
+        m[13] = __dadd_rn(m[13], fma(r2, s1, s3));
+    }
+}
+
 // FP64 raw moments {sum x, sum c x, sum |c|^2 x} of one row (block-wide)
 template <typename T, int VEC, int NVC = 0>
 __device__ __forceinline__ void row_moments(const T* __restrict__ row, int n, int Nv, const double* cs,
@@ -61,16 +129,7 @@ __device__ __forceinline__ void row_moments(const T* __restrict__ row, int n, in
         c.load(row + v);
         uint32_t ix, iy, iz;
         vsplit<NVC>(uint32_t(v), uint32_t(Nv), ix, iy, iz);
-        const double cx = cs[ix], cy = cs[iy], b = cx * cx + cy * cy;
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-            const double x = double(c.v[j]), cz = cs[iz + j];
-            m[0] += x;
-            m[1] += cx * x;
-            m[2] += cy * x;
-            m[3] += cz * x;
-            m[4] += (b + cz * cz) * x;
-        }
+        chunk_moments<T, VEC, 5>(c, cs[ix], cs[iy], cs + iz, m);
     }
 }
 
