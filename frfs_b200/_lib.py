@@ -28,6 +28,7 @@ EXPORTS = (
     'bdgfs_bgk_moments', 'bdgfs_bgk_maxwellian', 'bdgfs_ars_stage',
     'bdgfs_esbgk_moments', 'bdgfs_esbgk_gaussian', 'bdgfs_shakov_moments', 'bdgfs_shakov_target',
     'bdgfs_bdf_step', 'bdgfs_vss_scratch_bytes', 'bdgfs_vss_collide', 'bdgfs_vss_project',
+    'bdgfs_vss_pair_scratch_bytes', 'bdgfs_vss_pair_collide',
 )
 
 
@@ -119,6 +120,13 @@ class VssArgs(C.Structure):
                 ('sz', C.c_void_p), ('b', C.c_void_p), ('c', C.c_void_p)]
 
 
+class VssPairArgs(C.Structure):
+    _fields_ = [('Nv', C.c_int32), ('Nrho', C.c_int32), ('M', C.c_int32), ('pad_', C.c_int32),
+                ('ndof', C.c_int64), ('f', C.c_void_p * 2), ('Q', C.c_void_p * 2),
+                ('phase', C.c_void_p), ('bself', C.c_void_p), ('bcross', C.c_void_p),
+                ('c', C.c_void_p)]
+
+
 class VssProjArgs(C.Structure):
     _fields_ = [('Nv', C.c_int32), ('nspcs', C.c_int32), ('ndof', C.c_int64),
                 ('fp64', C.c_int32), ('pad_', C.c_int32), ('Q', C.c_void_p * 4),
@@ -194,6 +202,7 @@ def lib():
             'bdgfs_bdf_step': [vp, vp],
             'bdgfs_vss_scratch_bytes': [C.c_int32, C.c_int32, C.c_int32],
             'bdgfs_vss_collide': [vp, vp, C.c_size_t, vp],
+            'bdgfs_vss_pair_collide': [vp, vp, i64, vp],
             'bdgfs_vss_project': [vp, vp],
             'bdgfs_colsum': [vp, i64, i64, vp, vp],
             'bdgfs_wait_probe': [C.c_uint32, i32, vp, vp],
@@ -204,6 +213,8 @@ def lib():
             fn = getattr(L, name)
             fn.restype = C.c_int32
             fn.argtypes = at
+        L.bdgfs_vss_pair_scratch_bytes.restype = C.c_int64
+        L.bdgfs_vss_pair_scratch_bytes.argtypes = [C.c_int32]
         _lib = L
     return _lib
 

@@ -1614,7 +1614,7 @@ static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_
     if (fit < 1) return BDGFS_ESCRATCH;
     a.tickets = reinterpret_cast<uint32_t*>(base);
     a.slots = reinterpret_cast<unsigned char*>(base + (size_t(fit) * sizeof(uint32_t) + 255) / 256 * 256);
-    int64_t parts = std::min(a.g.Nrho, tree::kMaxSplit);
+    int64_t parts = std::min(a.g.Nrho, kMaxParts);
     if (!dev_count) parts = tree_split(total, fit, a.g.Nrho, nsm);
     if (parts > 1) {
         a.nslots = fit;

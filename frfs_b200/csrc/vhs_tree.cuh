@@ -48,6 +48,7 @@
 // two of the SM's sub-partitions, which caps registers at 168); the spectral
 // gain G^ in global scratch (L2), touched once per radius.
 #pragma once
+#include "split.cuh"
 
 namespace bdgfs {
 
@@ -61,7 +62,6 @@ constexpr int kMaxM = 48;                     // directions (node tables in shar
 constexpr int kGroups = (NT / 32 + 3) / 4;    // TMEM column groups
 constexpr uint32_t kAB = 0, kS = 4 * N * kGroups;   // TMEM columns: node pencils, S_p
 constexpr uint32_t kCols = 512;
-constexpr int kMaxSplit = 16;
 static_assert(NT >= NP && 2 * NT >= NZ && NT < NZ, "thread roles");
 static_assert(kS + 2 * N * kGroups <= kCols, "TMEM columns");
 }  // namespace tree
@@ -152,24 +152,12 @@ __device__ inline void tree_plan(const cpx<float>* phase, int Nrho, int M, TreeP
     }
 }
 
-// Parts that each distribution's radii are cut into: the split with the
-// smallest (rounds of CTAs) x (radii per part + the work every part repeats,
-// about 1.5 radii), so that short lists occupy the SMs and a nearly empty last
-// round costs a part of a distribution's time only.  97 distributions on 148
-// SMs: 3 parts, 0.349 ms against 0.44 ms uncut.
+// Parts that each distribution's radii are cut into (split.cuh); F and the final
+// transforms cost about 1.5 radii, the sum of the parts 0.2 more.  97
+// distributions on 148 SMs: 3 parts, 0.349 ms against 0.44 ms uncut.
 __host__ __device__ inline int tree_split(int64_t total, int64_t nslots, int Nrho, int ncta)
 {
-    int best = 1;
-    float cost = 1e30f;
-    for (int ns = 1; ns <= (Nrho < tree::kMaxSplit ? Nrho : tree::kMaxSplit); ++ns) {
-        if (ns > 1 && total * ns > nslots) break;
-        const float c = float((total * ns + ncta - 1) / ncta) * (float((Nrho + ns - 1) / ns) + (ns > 1 ? 1.7f : 1.5f));
-        if (c < 0.97f * cost) {
-            cost = c;
-            best = ns;
-        }
-    }
-    return best;
+    return split_parts(total, nslots, Nrho, ncta, 1.5f, 1.7f);
 }
 
 __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)

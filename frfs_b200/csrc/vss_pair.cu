@@ -1,0 +1,474 @@
+// Mixture VSS collision operator for two species at Nv = 24, FP32, with an
+// antipodal direction set: Q_p = sum_q Q_pq (vss.cu states the operator and the
+// reference).
+//
+// For a direction s and its opposite the slices repeat: with a -> -a the two
+// factors of T_pq(s) = IFFT(e^{+i mu_q a} F_p) IFFT(e^{-i mu_p a} F_q) are those of
+// T_qp, so T_qp(-s) = T_pq(s) and T_pp(-s) = T_pp(s), exactly.  One radius then
+// needs M/2 slices for each species with itself and M for the unlike pair,
+// whose transform feeds both gains, instead of 4 M; the kernel weights of s and
+// -s are added in the table (their sum is real: b(-s) = conj b(s)).
+//
+// One persistent CTA of 320 threads per distribution (or per range of radii of
+// one, when distributions are few).  A slice carries its two factors as the two
+// lanes of f32x2 numbers through the inverse passes x, y, z, multiplies them in
+// registers, and transforms the product z, y, x.  The exchange cube holds
+// (A.re, B.re, A.im, B.im) at (x*24 + y)*25 + z: every pass reads and writes its
+// own pencils in place, in 16-byte accesses free of bank conflicts; the product
+// goes into the same rows as 8-byte numbers, offset by one in every second
+// group of eight rows.  G^ of both species stays in tensor memory.  F comes from
+// the CTA's scratch and the weights from their tables, through L2: 165 KB (like
+// pair) or 442 KB a slice.  Measured on one B200, Nrho = M = 12, 370 argon-krypton
+// pairs: 25.5 -> 12.2 ms (the general kernel of vss.cu -> this one); error against
+// 64-bit arithmetic 4.2e-6 -> 4.9e-6 of Q.  Bound: the FP32 pipe and the barriers
+// between passes.  (The factors are real but for Nyquist terms; packing them as
+// one complex transform drops those terms, 1e-3 of Q on this mixture.)
+#include <algorithm>
+
+#include "common.cuh"
+#include "fft_codelets.cuh"
+#include "split.cuh"
+#include "tcgen05.cuh"
+
+namespace bdgfs {
+
+namespace vssp {
+constexpr int N = 24, n = N * N * N, NZ = N * N, NT = 320;
+constexpr int RP = N + 1, PX = N * RP;                       // pitches of y and x
+constexpr int kTask = 4 * N;                                 // TMEM columns of a task: G^ of both species
+constexpr size_t kCube = size_t(N) * PX * sizeof(float4);
+constexpr size_t kSmem = kCube + 3 * N * sizeof(float4);
+constexpr size_t kF = size_t(N) * NZ * sizeof(float4);       // F of both species
+constexpr size_t kSlot = size_t(N) * NZ * sizeof(float4);    // partial G^ of both species
+}  // namespace vssp
+
+struct VssPairArgs {
+    bdgfs_vss_pair_args g;
+    unsigned char* F;                // [CTA] kF
+    unsigned char* slots;            // [item] kSlot (split launches)
+    uint32_t* tickets;               // [distribution], zeroed (split launches)
+    int32_t ns;                      // parts per distribution
+    uint32_t* timeout;               // set when a bounded wait ran out
+};
+
+__device__ __forceinline__ float2 v2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+
+__global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs a)
+{
+    using namespace vssp;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_last;
+    __shared__ __align__(8) uint64_t s_free;
+    const bdgfs_vss_pair_args& g = a.g;
+    float4* W = reinterpret_cast<float4*>(smem);
+    float2* T = reinterpret_cast<float2*>(smem);
+    float4* E = W + N * PX;                                    // [axis][k]: (E1.re, E2.re, E1.im, E2.im)
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (tid < 32) tc::tmem_alloc(&s_tmem, 512);
+    if (tid == 0) tc::mbar_init(&s_free, NT);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    // task r of the thread: pencil tid + r * 320; warps 0-7 have two (their
+    // TMEM columns 0..191 or 192..383), warps 8 and 9 one (384..479)
+    const int ntask = tid + NT < NZ ? 2 : 1;
+    const uint32_t tcol = s_tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(2 * kTask * (warp >> 2));
+
+    uint32_t par = 1;
+    bool dead = false;                                          // a wait ran out: finish without waiting again
+    auto wait_free = [&]() {
+        for (uint32_t spins = 0; !dead && !tc::mbar_try(&s_free, par);) {
+            if (++spins == (1u << 22)) {
+                dead = true;
+                atomicOr(a.timeout, 1u);
+            }
+        }
+        par ^= 1u;
+        __syncwarp();
+    };
+    auto arrive = [&]() { tc::mbar_arrive(&s_free); };
+    // cube addresses: pencil t = i * 24 + j of each pass
+    auto at_x = [](int t) { return (t / N) * RP + t % N; };            // (y, z): + x * PX
+    auto at_y = [](int t) { return (t / N) * PX + t % N; };            // (x, z): + y * RP
+    auto at_z = [](int t) { return (t / N) * PX + (t % N) * RP; };     // (x, y): + z
+    auto t_row = [](int x, int y) { return 2 * (x * PX + y * RP) + ((3 * x + (y >> 3)) & 1); };  // product: + z
+    auto get = [&](int b, int s, float2 (&vr)[N], float2 (&vi)[N]) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float4 v = W[b + k * s];
+            vr[k] = v2(v.x, v.y);
+            vi[k] = v2(v.z, v.w);
+        }
+    };
+    auto put = [&](int b, int s, const float2 (&vr)[N], const float2 (&vi)[N]) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) W[b + k * s] = make_float4(vr[k].x, vr[k].y, vi[k].x, vi[k].y);
+    };
+    auto pass_y_inv = [&]() {
+#pragma unroll 1
+        for (int r = 0; r < ntask; ++r) {
+            const int b = at_y(tid + r * NT);
+            float2 vr[N], vi[N];
+            get(b, RP, vr, vi);
+            dft_p2<N, +1>(vr, vi);
+            put(b, RP, vr, vi);
+        }
+    };
+
+    float4* F = reinterpret_cast<float4*>(a.F + size_t(blockIdx.x) * kF);      // [kx][ky*24 + kz]: (F0.re, F1.re, F0.im, F1.im)
+    const int Nrho = g.Nrho, M = g.M, ns = a.ns;
+    const float4* phase = static_cast<const float4*>(g.phase);
+    const float* bself = static_cast<const float*>(g.bself);
+    const float4* bcross = static_cast<const float4*>(g.bcross);
+    const float2* c = static_cast<const float2*>(g.c);
+    const int64_t nitems = g.ndof * ns;
+    for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const int64_t dof = item / ns;
+        const int part = int(item - dof * ns);
+        const float* f0 = static_cast<const float*>(g.f[0]) + dof * n;
+        const float* f1 = static_cast<const float*>(g.f[1]) + dof * n;
+
+        // ---- F_p = FFT(f_p) / n, both species ----
+        wait_free();
+#pragma unroll 1
+        for (int r = 0; r < ntask; ++r) {
+            const int t = tid + r * NT;
+            float2 vr[N], vi[N];
+#pragma unroll
+            for (int z = 0; z < N; ++z) {
+                vr[z] = v2(f0[t * N + z], f1[t * N + z]);
+                vi[z] = v2(0.f, 0.f);
+            }
+            dft_p2<N, -1>(vr, vi);
+            put(at_z(t), 1, vr, vi);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int r = 0; r < ntask; ++r) {
+            const int b = at_y(tid + r * NT);
+            float2 vr[N], vi[N];
+            get(b, RP, vr, vi);
+            dft_p2<N, -1>(vr, vi);
+            put(b, RP, vr, vi);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int r = 0; r < ntask; ++r) {
+            const int t = tid + r * NT;
+            float2 vr[N], vi[N];
+            get(at_x(t), PX, vr, vi);
+            if (r + 1 == ntask) arrive();
+            dft_p2<N, -1>(vr, vi);
+            const float sc = 1.f / float(n);
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                F[k * NZ + t] = make_float4(vr[k].x * sc, vr[k].y * sc, vi[k].x * sc, vi[k].y * sc);
+            uint32_t zero[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) zero[k] = 0u;
+#pragma unroll
+            for (int k = 0; k < kTask / 16; ++k) tc::tmem_st16(tcol + r * kTask + 16 * k, zero);
+        }
+        tc::tmem_wait_st();
+
+        // ---- slices: radius rho, pair kind (0: species 0 with itself, 1: species 1
+        // with itself, 2: unlike), direction s; phase tables kind by kind ----
+        const int rho1 = Nrho * (part + 1) / ns;
+        int rho = Nrho * part / ns, kind = 0, s = 0;
+        const int half = M / 2;
+        auto table = [&](int q, int k, int d) { return (k < 2 ? (k * Nrho + q) * half : (Nrho + q) * M) + d; };
+        if (tid < 3 * N) E[tid] = phase[size_t(table(rho, 0, 0)) * 3 * N + tid];
+        __syncthreads();
+        while (rho < rho1) {
+            const int ti = table(rho, kind, s);
+            // the slice after this one
+            int nrho = rho, nkind = kind, ndir = s + 1;
+            if (ndir == (kind < 2 ? half : M)) {
+                ndir = 0;
+                if (++nkind == 3) {
+                    nkind = 0;
+                    ++nrho;
+                }
+            }
+            float4 enext = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid < 3 * N && nrho < rho1) enext = phase[size_t(table(nrho, nkind, ndir)) * 3 * N + tid];
+            // x: phases and inverse transform
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT;
+                const float4 ey = E[N + t / N], ez = E[2 * N + t % N];
+                const float2 yr = v2(ey.x, ey.y), yi = v2(ey.z, ey.w), zr = v2(ez.x, ez.y), zi = v2(ez.z, ez.w);
+                const float2 er = __ffma2_rn(neg2(yi), zi, __fmul2_rn(yr, zr));
+                const float2 ei = __ffma2_rn(yr, zi, __fmul2_rn(yi, zr));
+                const float2 nei = neg2(ei);
+                float2 vr[N], vi[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const float4 v = F[k * NZ + t];
+                    vr[k] = v2(kind == 1 ? v.y : v.x, kind == 0 ? v.x : v.y);
+                    vi[k] = v2(kind == 1 ? v.w : v.z, kind == 0 ? v.z : v.w);
+                }
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const float4 x = E[k];
+                    const float2 xr = v2(x.x, x.y), xi = v2(x.z, x.w);
+                    const float2 cr = __ffma2_rn(xi, nei, __fmul2_rn(xr, er));
+                    const float2 ci = __ffma2_rn(xi, er, __fmul2_rn(xr, ei));
+                    const float2 re = __ffma2_rn(neg2(ci), vi[k], __fmul2_rn(cr, vr[k]));
+                    vi[k] = __ffma2_rn(ci, vr[k], __fmul2_rn(cr, vi[k]));
+                    vr[k] = re;
+                }
+                dft_p2<N, +1>(vr, vi);
+                if (r == 0) wait_free();
+                put(at_x(t), PX, vr, vi);
+            }
+            __syncthreads();
+            if (tid < 3 * N) E[tid] = enext;                    // read after the next barriers
+            pass_y_inv();
+            __syncthreads();
+            // z: inverse transform, product, forward transform
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT;
+                cpx<float> X[N];
+                {
+                    float2 vr[N], vi[N];
+                    get(at_z(t), 1, vr, vi);
+                    dft_p2<N, +1>(vr, vi);
+#pragma unroll
+                    for (int z = 0; z < N; ++z)
+                        X[z] = {fmaf(vr[z].x, vr[z].y, -vi[z].x * vi[z].y), fmaf(vr[z].x, vi[z].y, vi[z].x * vr[z].y)};
+                }
+                dft<N, -1>(X);
+                const int b = t_row(t / N, t % N);
+#pragma unroll
+                for (int k = 0; k < N; ++k) T[b + k] = v2(X[k].x, X[k].y);
+            }
+            __syncthreads();
+            // y: forward transform of the product
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT, x = t / N, z = t % N;
+                cpx<float> X[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const float2 v = T[t_row(x, k) + z];
+                    X[k] = {v.x, v.y};
+                }
+                dft<N, -1>(X);
+#pragma unroll
+                for (int k = 0; k < N; ++k) T[t_row(x, k) + z] = v2(X[k].x, X[k].y);
+            }
+            __syncthreads();
+            // x: forward transform, weighted into G^
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT, y = t / N, z = t % N;
+                cpx<float> X[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const float2 v = T[t_row(k, y) + z];
+                    X[k] = {v.x, v.y};
+                }
+                if (r + 1 == ntask) arrive();
+                dft<N, -1>(X);
+                tc::tmem_wait_st();
+                const uint32_t col = tcol + r * kTask;
+                if (kind < 2) {
+                    const float* w = bself + size_t(ti) * n + t;
+#pragma unroll
+                    for (int cc = 0; cc < N / 8; ++cc) {
+                        float b[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) b[k] = ldg(w + (8 * cc + k) * NZ);
+                        uint32_t u[16];
+                        tc::tmem_ld16_issue(col + kind * 2 * N + 16 * cc, u);
+                        tc::tmem_wait();
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const cpx<float> x = X[8 * cc + k];
+                            u[2 * k] = __float_as_uint(fmaf(b[k], x.x, __uint_as_float(u[2 * k])));
+                            u[2 * k + 1] = __float_as_uint(fmaf(b[k], x.y, __uint_as_float(u[2 * k + 1])));
+                        }
+                        tc::tmem_st16(col + kind * 2 * N + 16 * cc, u);
+                    }
+                } else {
+                    const float4* w = bcross + size_t(ti - Nrho * M) * n + t;
+#pragma unroll
+                    for (int cc = 0; cc < N / 8; ++cc) {
+                        float4 b[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) b[k] = __ldg(w + (8 * cc + k) * NZ);
+                        uint32_t u[16], q[16];
+                        tc::tmem_ld16_issue(col + 16 * cc, u);
+                        tc::tmem_ld16_issue(col + 2 * N + 16 * cc, q);
+                        tc::tmem_wait();
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const cpx<float> x = X[8 * cc + k];
+                            const float4 v = b[k];
+                            u[2 * k] = __float_as_uint(fmaf(v.x, x.x, fmaf(-v.y, x.y, __uint_as_float(u[2 * k]))));
+                            u[2 * k + 1] = __float_as_uint(fmaf(v.x, x.y, fmaf(v.y, x.x, __uint_as_float(u[2 * k + 1]))));
+                            q[2 * k] = __float_as_uint(fmaf(v.z, x.x, fmaf(-v.w, x.y, __uint_as_float(q[2 * k]))));
+                            q[2 * k + 1] = __float_as_uint(fmaf(v.z, x.y, fmaf(v.w, x.x, __uint_as_float(q[2 * k + 1]))));
+                        }
+                        tc::tmem_st16(col + 16 * cc, u);
+                        tc::tmem_st16(col + 2 * N + 16 * cc, q);
+                    }
+                }
+            }
+            rho = nrho;
+            kind = nkind;
+            s = ndir;
+        }
+        tc::tmem_wait_st();
+
+        const float4* sum = nullptr;                            // parts' G^, when split
+        if (ns > 1) {
+            float4* slot = reinterpret_cast<float4*>(a.slots + size_t(item) * kSlot);
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+#pragma unroll
+                for (int cc = 0; cc < N / 8; ++cc) {
+                    uint32_t u[16], q[16];
+                    tc::tmem_ld16_issue(tcol + r * kTask + 16 * cc, u);
+                    tc::tmem_ld16_issue(tcol + r * kTask + 2 * N + 16 * cc, q);
+                    tc::tmem_wait();
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        __stcg(slot + (8 * cc + k) * NZ + tid + r * NT,
+                               make_float4(__uint_as_float(u[2 * k]), __uint_as_float(u[2 * k + 1]),
+                                           __uint_as_float(q[2 * k]), __uint_as_float(q[2 * k + 1])));
+                }
+            }
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(a.tickets + dof, 1u) == uint32_t(ns - 1);
+            __syncthreads();
+            if (!s_last) continue;
+            __threadfence();
+            sum = reinterpret_cast<const float4*>(a.slots + size_t(dof) * ns * kSlot);
+        }
+
+        // ---- back to velocity space: lane A QG_p, lane B QL_p; Q_p = QG_p - f_p QL_p ----
+#pragma unroll 1
+        for (int p = 0; p < 2; ++p) {
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT;
+                float2 vr[N], vi[N];
+                if (sum) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) vr[k].x = vi[k].x = 0.f;
+#pragma unroll 1
+                    for (int j = 0; j < ns; ++j) {
+                        const float2* sj = reinterpret_cast<const float2*>(sum + size_t(j) * N * NZ);
+#pragma unroll
+                        for (int k = 0; k < N; ++k) {
+                            const float2 v = __ldcg(sj + 2 * (k * NZ + t) + p);
+                            vr[k].x += v.x;
+                            vi[k].x += v.y;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int cc = 0; cc < N / 8; ++cc) {
+                        uint32_t u[16];
+                        tc::tmem_ld16_issue(tcol + r * kTask + p * 2 * N + 16 * cc, u);
+                        tc::tmem_wait();
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            vr[8 * cc + k].x = __uint_as_float(u[2 * k]);
+                            vi[8 * cc + k].x = __uint_as_float(u[2 * k + 1]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const float4 v = F[k * NZ + t];
+                    const float2 ca = __ldg(c + size_t(2 * p) * n + k * NZ + t);
+                    const float2 cb = __ldg(c + size_t(2 * p + 1) * n + k * NZ + t);
+                    vr[k].y = ca.x * v.x - ca.y * v.z + cb.x * v.y - cb.y * v.w;
+                    vi[k].y = ca.x * v.z + ca.y * v.x + cb.x * v.w + cb.y * v.y;
+                }
+                dft_p2<N, +1>(vr, vi);
+                if (r == 0) wait_free();
+                put(at_x(t), PX, vr, vi);
+            }
+            __syncthreads();
+            pass_y_inv();
+            __syncthreads();
+            const float* fp = p ? f1 : f0;
+            float* Q = static_cast<float*>(g.Q[p]) + dof * n;
+#pragma unroll 1
+            for (int r = 0; r < ntask; ++r) {
+                const int t = tid + r * NT;
+                float2 vr[N], vi[N];
+                get(at_z(t), 1, vr, vi);
+                if (r + 1 == ntask) arrive();
+                dft_p2<N, +1>(vr, vi);
+#pragma unroll
+                for (int z = 0; z < N; ++z) Q[t * N + z] = vr[z].x - fp[t * N + z] * vr[z].y;
+            }
+        }
+    }
+    tc::tmem_wait_st();
+    tc::tc_fence_before();
+    __syncthreads();
+    if (tid < 32) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(s_tmem, 512);
+    }
+}
+
+}  // namespace bdgfs
+
+using namespace bdgfs;
+
+// scratch: [timeout word, tickets, padding][F per CTA][slots]
+static size_t vssp_head(int64_t nslots) { return (size_t(nslots + 1) * sizeof(uint32_t) + 255) / 256 * 256; }
+
+extern "C" int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas)
+{
+    if (nctas < 1) return 0;
+    // one F and two slots per CTA
+    return int64_t(vssp_head(2 * int64_t(nctas)) + size_t(nctas) * (vssp::kF + 2 * vssp::kSlot) + 256);
+}
+
+extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* scratch, int64_t bytes, void* stream)
+{
+    using namespace vssp;
+    if (!g || !scratch || g->ndof < 0 || g->Nrho < 1 || g->M < 2 || g->M % 2 || !g->phase || !g->bself || !g->bcross ||
+        !g->c || !g->f[0] || !g->f[1] || !g->Q[0] || !g->Q[1])
+        return BDGFS_EINVAL;
+    if (g->Nv != N) return BDGFS_EUNSUPPORTED;
+    if (g->ndof == 0) return BDGFS_OK;
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return BDGFS_ECUDA;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return BDGFS_ECUDA;
+    // CTAs and slots that fit
+    const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
+    const int64_t room = bytes - int64_t(base - reinterpret_cast<uintptr_t>(scratch));
+    int64_t nctas = std::min<int64_t>(nsm, (room - int64_t(vssp_head(0))) / int64_t(kF));
+    if (nctas < 1) return BDGFS_ESCRATCH;
+    int64_t nslots = 0;
+    while (int64_t(vssp_head(nslots + 1) + size_t(nctas) * kF + size_t(nslots + 1) * kSlot) <= room &&
+           nslots < 4 * int64_t(nsm))
+        ++nslots;
+    VssPairArgs a{};
+    a.g = *g;
+    a.ns = split_parts(g->ndof, nslots, g->Nrho, int(nctas), 0.3f, 0.4f);
+    a.timeout = reinterpret_cast<uint32_t*>(base);
+    a.tickets = a.timeout + 1;
+    a.F = reinterpret_cast<unsigned char*>(base + vssp_head(nslots));
+    a.slots = a.F + size_t(nctas) * kF;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(a.timeout, 0, sizeof(uint32_t) * (1 + (a.ns > 1 ? size_t(g->ndof) : 0)), st) != cudaSuccess)
+        return BDGFS_ECUDA;
+    if (const int rc = smem_optin(reinterpret_cast<const void*>(vss_pair_kernel), kSmem)) return rc;
+    nctas = std::min(nctas, g->ndof * a.ns);
+    vss_pair_kernel<<<unsigned(nctas), NT, kSmem, st>>>(a);
+    return cuda_status(cudaGetLastError());
+}

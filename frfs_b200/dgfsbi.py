@@ -208,15 +208,18 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         dev = be.device
         S, n = self._nspcs, vm.vsize()
         self.fp64 = int(be.fpdtype == torch.float64)
-        ct = torch.complex128 if self.fp64 else torch.complex64
         m = vm.masses()
-        b = torch.empty((S * S, vm.Nrho() * vm.M(), n), dtype=ct, device=dev)
-        c = torch.empty((S * S, n), dtype=ct, device=dev)
-        for p, q in self._cases:
-            bb, cc = self.kernel_tables(p, q)
-            b[p * S + q].copy_(torch.from_numpy(bb))
-            c[p * S + q].copy_(torch.from_numpy(cc))
-        self.d_b, self.d_c = b, c
+        tables = {(p, q): self.kernel_tables(p, q) for p, q in self._cases}
+        self._pair = self._pair_tables(tables)
+        if self._pair is None:
+            ct = torch.complex128 if self.fp64 else torch.complex64
+            b = torch.empty((S * S, vm.Nrho() * vm.M(), n), dtype=ct, device=dev)
+            c = torch.empty((S * S, n), dtype=ct, device=dev)
+            for (p, q), (bb, cc) in tables.items():
+                b[p * S + q].copy_(torch.from_numpy(bb))
+                c[p * S + q].copy_(torch.from_numpy(cc))
+            self.d_b, self.d_c = b, c
+        del tables
         f64 = lambda a: torch.as_tensor(np.asarray(a, np.float64), device=dev).contiguous()
         self.d_mfrac = f64([m[q] / (m[p] + m[q]) for p, q in self._cases])
         self.d_prefac = f64([self._prefactor[f'{p}{q}'] for p, q in self._cases])
@@ -224,7 +227,7 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         self.d_rw = f64(vm.qw() * vm.sw() / n)
         self.d_sz = f64(vm.sz())
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == 'cuda' else 1
-        self._nctas = nsm
+        self._nctas = nsm                              # CTAs that scratch is kept for
         self._scratch = None
         # FP64 conservation projection (species masses, total momentum and
         # energy); the reference's operator has none, so parity runs disable it
@@ -232,6 +235,57 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         self.d_c0 = f64(vm.c0())
         self.d_mass = f64(m)
         self.d_ginv = f64(mixture_gram_inverse(vm.c0(), m).ravel())
+
+    def _pair_tables(self, tables):
+        """Tables of ``bdgfs_vss_pair_collide`` (two species, Nv = 24, FP32),
+        or None where that kernel does not apply: it needs direction M/2 + s
+        to be the opposite of s, and b(-s) = conj b(s) (an antipodal
+        pre-computation sphere)."""
+        vm, dev = self.vm, self.backend.device
+        Nrho, M, n, N = vm.Nrho(), vm.M(), vm.vsize(), vm.Nv()
+        sz, h = np.asarray(vm.sz()), vm.M() // 2
+        if self._nspcs != 2 or self.fp64 or N != 24 or M % 2 or not np.array_equal(sz[h:], -sz[:h]):
+            return None
+        w = (vm.qw() * vm.sw() / n)[:, None, None]
+        bself = torch.empty((2, Nrho, h, n), dtype=torch.float32, device=dev)
+        bcross = torch.empty((Nrho, M, n, 4), dtype=torch.float32, device=dev)
+        for p in (0, 1):
+            b = tables[p, p][0].reshape(Nrho, M, n)
+            both = b[:, :h] + b[:, h:]
+            if np.abs(both.imag).max() > 1e-12 * np.abs(b).max():
+                return None
+            bself[p].copy_(torch.from_numpy(self._prefactor[f'{p}{p}'] * w * both.real))
+        # b_10(-s): the halves swapped
+        b10 = tables[1, 0][0].reshape(Nrho, M, n)
+        b10 = np.concatenate([b10[:, h:], b10[:, :h]], axis=1)
+        for k, (pq, b) in enumerate((('01', tables[0, 1][0].reshape(Nrho, M, n)), ('10', b10))):
+            b = np.ascontiguousarray(self._prefactor[pq] * w * b).view(np.float64).reshape(Nrho, M, n, 2)
+            bcross[..., 2 * k:2 * k + 2].copy_(torch.from_numpy(b))
+        c = np.stack([self._prefactor[f'{p}{q}'] * tables[p, q][1] for p, q in self._cases])
+        # phases exp(i mu a_d l), exp(-i mu' a_d l) of every slice, axis and l
+        l0 = np.concatenate((np.arange(0, N // 2), np.arange(-N // 2, 0))).astype(np.float64)
+        m = vm.masses()
+        mu1 = m[1] / (m[0] + m[1])
+        a = (np.pi / vm.L() * vm.qz())[:, None, None, None] * sz[None, :, :, None] * l0       # [Nrho][M][3][N]
+        ph = lambda x, y: np.stack([np.cos(x), np.cos(y), np.sin(x), np.sin(y)], axis=-1)
+        like = ph(0.5 * a[:, :h], -0.5 * a[:, :h]).reshape(-1, 3, N, 4)
+        phase = np.concatenate([like, like, ph(mu1 * a, -(1.0 - mu1) * a).reshape(-1, 3, N, 4)])
+        f32 = lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(torch.float32).to(dev)
+        return dict(bself=bself, bcross=bcross, phase=f32(phase),
+                    c=torch.from_numpy(c).to(torch.complex64).to(dev).contiguous())
+
+    def _collide_pair(self, fs, Qs, ndof):
+        t, L = self._pair, _lib.lib()
+        a = _lib.VssPairArgs(Nv=self.vm.Nv(), Nrho=self.vm.Nrho(), M=self.vm.M(), ndof=ndof,
+                             phase=t['phase'].data_ptr(), bself=t['bself'].data_ptr(),
+                             bcross=t['bcross'].data_ptr(), c=t['c'].data_ptr())
+        for p in (0, 1):
+            a.f[p], a.Q[p] = fs[p].data_ptr(), Qs[p].data_ptr()
+        nb = L.bdgfs_vss_pair_scratch_bytes(self._nctas)
+        if self._scratch is None or self._scratch.numel() < nb:
+            self._scratch = torch.empty(nb, dtype=torch.uint8, device=self.backend.device)
+        _lib.check(L.bdgfs_vss_pair_collide(C.byref(a), self._scratch.data_ptr(), nb, _lib.stream_ptr()),
+                   'bdgfs_vss_pair_collide')
 
     def _scratch_for(self, items):
         L = _lib.lib()
@@ -250,18 +304,22 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         if len(fs) != S or len(Qs) != S:
             raise ValueError(f'need {S} species banks')
         ndof = fs[0].numel() // n
-        a = _lib.VssArgs(Nv=self.vm.Nv(), nspcs=S, Nrho=self.vm.Nrho(), M=self.vm.M(),
-                         ndof=ndof, fp64=self.fp64, mfrac=self.d_mfrac.data_ptr(),
-                         prefac=self.d_prefac.data_ptr(), rfac=self.d_rfac.data_ptr(),
-                         rw=self.d_rw.data_ptr(), sz=self.d_sz.data_ptr(), b=self.d_b.data_ptr(),
-                         c=self.d_c.data_ptr())
         for p in range(S):
             if fs[p].numel() != ndof * n or Qs[p].numel() != ndof * n:
                 raise ValueError('species banks must hold the same distributions')
-            a.f[p], a.Q[p] = fs[p].data_ptr(), Qs[p].data_ptr()
-        scratch, nb = self._scratch_for(ndof * S)
-        _lib.check(_lib.lib().bdgfs_vss_collide(C.byref(a), scratch.data_ptr(), nb,
-                                                _lib.stream_ptr()), 'bdgfs_vss_collide')
+        if self._pair is not None:
+            self._collide_pair(fs, Qs, ndof)
+        else:
+            a = _lib.VssArgs(Nv=self.vm.Nv(), nspcs=S, Nrho=self.vm.Nrho(), M=self.vm.M(),
+                             ndof=ndof, fp64=self.fp64, mfrac=self.d_mfrac.data_ptr(),
+                             prefac=self.d_prefac.data_ptr(), rfac=self.d_rfac.data_ptr(),
+                             rw=self.d_rw.data_ptr(), sz=self.d_sz.data_ptr(), b=self.d_b.data_ptr(),
+                             c=self.d_c.data_ptr())
+            for p in range(S):
+                a.f[p], a.Q[p] = fs[p].data_ptr(), Qs[p].data_ptr()
+            scratch, nb = self._scratch_for(ndof * S)
+            _lib.check(_lib.lib().bdgfs_vss_collide(C.byref(a), scratch.data_ptr(), nb,
+                                                    _lib.stream_ptr()), 'bdgfs_vss_collide')
         if self._project if project is None else project:
             pa = _lib.VssProjArgs(Nv=self.vm.Nv(), nspcs=S, ndof=ndof, fp64=self.fp64,
                                   c0=self.d_c0.data_ptr(), mass=self.d_mass.data_ptr(),

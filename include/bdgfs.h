@@ -545,6 +545,34 @@ size_t bdgfs_vss_scratch_bytes(int32_t Nv, int32_t fp64, int32_t nctas);
 int32_t bdgfs_vss_collide(const bdgfs_vss_args* a, void* scratch, size_t bytes,
                           void* stream);
 
+/* The same operator for two species at Nv = 24, FP32, with an antipodal
+ * direction set (direction M/2 + s is the opposite of s): the slices of s and
+ * -s coincide (T_qp(-s) = T_pq(s)), so a radius needs M/2 slices for each like
+ * pair and M for the unlike one.  The caller passes the weights of a slice
+ * already multiplied by prefac_pq qw_r sw / n and, for like pairs, added over s
+ * and -s (their sum is real). */
+typedef struct bdgfs_vss_pair_args {
+    int32_t Nv, Nrho, M, pad_;
+    int64_t ndof;
+    const void* f[2];        /* float [ndof][n]                              */
+    void* Q[2];              /* float [ndof][n]                              */
+    const void* phase;       /* float4 [2 Nrho M][3][Nv]: per slice and axis
+                                (Re E1, Re E2, Im E1, Im E2) with
+                                E1 = exp(i mu_q a_d l), E2 = exp(-i mu_p a_d l);
+                                slices: pair 00 [Nrho][M/2], 11 [Nrho][M/2],
+                                01 [Nrho][M]                                 */
+    const void* bself;       /* float [Nrho M][n]: pairs 00 then 11          */
+    const void* bcross;      /* float4 [Nrho M][n]: (Re, Im) of b_01(s) and of
+                                b_10(-s)                                     */
+    const void* c;           /* complex float [4][n]: prefac_pq c_pq         */
+} bdgfs_vss_pair_args;
+
+/* Bytes of device scratch for nctas CTAs (one per SM runs every launch at full
+ * speed; less runs fewer CTAs, below one CTA's BDGFS_ESCRATCH). */
+int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas);
+int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* a, void* scratch,
+                               int64_t bytes, void* stream);
+
 /* FP64 conservation projection of a mixture's Q, in place, per
  * distribution: the minimal-norm change of (Q_0 .. Q_{S-1}) that zeroes each
  * species' mass and the total momentum and energy (species weighted by

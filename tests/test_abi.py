@@ -41,6 +41,7 @@ STRUCTS = {
     'bdgfs_bdf_args': _lib.BdfArgs,
     'bdgfs_vss_args': _lib.VssArgs,
     'bdgfs_vss_proj_args': _lib.VssProjArgs,
+    'bdgfs_vss_pair_args': _lib.VssPairArgs,
 }
 
 
