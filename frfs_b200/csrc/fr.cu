@@ -23,7 +23,9 @@
 // its own outward normal), which equals the reference's lhs-computed value
 // with the sign flip of intcflux.mako:21-23.
 #include "common.cuh"
+#include "fr_common.cuh"
 #include "fr_tc.cuh"
+#include "rows.cuh"
 
 namespace bdgfs {
 
@@ -32,54 +34,6 @@ struct FrSmem {
     T* dT;      // [ND*NU][NU]  (M1 - M3 M2) transposed
     T* m3T;     // [NF][NU]
     T* m0;      // [NF][NU]
-};
-
-// velocity components of index v
-template <typename T>
-__device__ __forceinline__ void vel(const T* c0, int Nv, int64_t v, T (&c)[3])
-{
-    // v < Nv^3 <= 2^18: 32-bit arithmetic
-    const uint32_t vv = uint32_t(v), n = uint32_t(Nv);
-    const uint32_t q = vv / n, iz = vv - q * n;
-    const uint32_t ix = q / n, iy = q - ix * n;
-    c[0] = c0[ix];
-    c[1] = c0[iy];
-    c[2] = c0[iz];
-}
-
-// VB consecutive values of a velocity row (one vector access when aligned)
-template <typename T, int VB>
-struct Vec {
-    T v[VB];
-    __device__ __forceinline__ void load(const T* __restrict__ p)
-    {
-        if constexpr (VB == 4 && sizeof(T) == 4) {
-            const float4 x = *reinterpret_cast<const float4*>(p);
-            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-        } else if constexpr (VB == 2 && sizeof(T) == 4) {
-            const float2 x = *reinterpret_cast<const float2*>(p);
-            v[0] = x.x; v[1] = x.y;
-        } else if constexpr (VB == 2 && sizeof(T) == 8) {
-            const double2 x = *reinterpret_cast<const double2*>(p);
-            v[0] = x.x; v[1] = x.y;
-        } else {
-#pragma unroll
-            for (int q = 0; q < VB; ++q) v[q] = p[q];
-        }
-    }
-    __device__ __forceinline__ void store(T* __restrict__ p) const
-    {
-        if constexpr (VB == 4 && sizeof(T) == 4) {
-            *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-        } else if constexpr (VB == 2 && sizeof(T) == 4) {
-            *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-        } else if constexpr (VB == 2 && sizeof(T) == 8) {
-            *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < VB; ++q) p[q] = v[q];
-        }
-    }
 };
 
 // r[0..N) = p[0..N) from shared memory in one vector load (p aligned to
@@ -266,21 +220,6 @@ __global__ void __launch_bounds__(128) disu_kernel(const bdgfs_fr_eles el, const
 // (tp.m1line, TPP nonzeros per column at compile-time rows) and M2 a
 // selection (row f: tp.fsgn[f] at column tp.fdim[f]*NU + fsel[f]), instead of
 // the dense M1 - M3 M2.
-// first velocity of the chunk of VB velocities that holds the mirror
-// images of v0 .. v0 + VB - 1 under c_d -> -c_d (the grid is symmetric:
-// c0[Nv - 1 - i] = -c0[i]); for the z axis the chunk holds them reversed.
-// Chunks never straddle a z line (VB divides Nv when a y or z mirror is
-// in use, checked on the host).
-__device__ __forceinline__ int64_t mirror_chunk(int64_t v0, int Nv, int kind, int VB)
-{
-    const int64_t N = Nv, N2 = N * N;
-    if (kind == BDGFS_BC_SPECULAR_X) return v0 + (N - 1 - 2 * (v0 / N2)) * N2;
-    if (kind == BDGFS_BC_SPECULAR_Y) return v0 + (N - 1 - 2 * ((v0 / N) % N)) * N;
-    const int64_t iz = v0 % N;
-    return v0 - iz + (N - iz - VB);
-}
-
-
 template <typename T, int ND, int NU, int NF, int VB, bool GATHER = false, int RING = 8, int TPP = 0>
 __global__ void __launch_bounds__(128, (NU <= 16 && sizeof(T) == 4) ? 4 : 3) rhs_kernel(const bdgfs_fr_eles el, const bdgfs_fr_walls wl,
                                                   const T* __restrict__ u, const T* __restrict__ uf,
@@ -600,14 +539,19 @@ __global__ void __launch_bounds__(128, (NU <= 16 && sizeof(T) == 4) ? 4 : 3) rhs
 }
 
 // uf: face-value rows [E][NF]; or, with fsel, the solution-point rows of u
-// ([E][NU]) read at row fsel[f] (GATHER, M0 rows unit vectors)
+// ([E][NU]) read at row fsel[f] (GATHER, M0 rows unit vectors).
+// One CTA per wall face point.  Bound by latency: few CTAs, two rows each.  So
+// a thread has two chunks of both rows in flight, its velocity index moves by
+// carries, the normal is padded to three components, and meshes with few wall
+// points get 1024 threads a row (bc_update_threads).  24^3 FP32 on one B200: 1926
+// points 76 -> 34 us, 256 points 16.7 -> 6.3 us, 84 points 14.1 -> 5.3 us.
 template <typename T>
-__global__ void __launch_bounds__(256) bc_update_kernel(const bdgfs_fr_eles el,
-                                                        const bdgfs_fr_walls wl,
-                                                        const T* __restrict__ uf,
-                                                        const int32_t* __restrict__ fsel)
+__global__ void __launch_bounds__(1024) bc_update_kernel(const bdgfs_fr_eles el,
+                                                         const bdgfs_fr_walls wl,
+                                                         const T* __restrict__ uf,
+                                                         const int32_t* __restrict__ fsel)
 {
-    __shared__ double red[2 * 8];
+    __shared__ double red[2 * 32];
     __shared__ T cs[1024];                                    // cell-centre velocities (Nv <= 1024)
     const int w = blockIdx.x;
     const int e = wl.fpt[2 * w], f = wl.fpt[2 * w + 1];
@@ -620,52 +564,57 @@ __global__ void __launch_bounds__(256) bc_update_kernel(const bdgfs_fr_eles el,
         }
         return;
     }
-    const int ND = el.ndims;
-    const T* pn = static_cast<const T*>(el.pnorm) + (int64_t(e) * el.nfpts + f) * ND;
-    const T* uw = static_cast<const T*>(wl.uwall) + bid * 3;
-    const T* fw = static_cast<const T*>(wl.fw) + int64_t(bid) * el.nv;
-    const T* ul = fsel ? uf + (int64_t(e) * el.nupts + fsel[f]) * el.nv
-                       : uf + (int64_t(e) * el.nfpts + f) * el.nv;
+    const int ND = el.ndims, Nv = el.Nv;
+    const T* gp = static_cast<const T*>(el.pnorm) + (int64_t(e) * el.nfpts + f) * ND;
+    const T* gu = static_cast<const T*>(wl.uwall) + bid * 3;
+    T pn[3], uw[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        pn[d] = d < ND ? gp[d] : T(0);
+        uw[d] = gu[d];
+    }
+    const T* __restrict__ fw = static_cast<const T*>(wl.fw) + int64_t(bid) * el.nv;
+    const T* __restrict__ ul = fsel ? uf + (int64_t(e) * el.nupts + fsel[f]) * el.nv
+                                    : uf + (int64_t(e) * el.nfpts + f) * el.nv;
     const T* c0 = static_cast<const T*>(el.c0);
-    for (int i = threadIdx.x; i < el.Nv; i += blockDim.x) cs[i] = c0[i];
+    for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = c0[i];
     __syncthreads();
     double s0 = 0.0, s1 = 0.0;
-    // four velocities per step (16-byte loads) when rows are aligned; with
-    // Nv % 4 == 0 the four share one z line (one index split per step)
-    const bool v4 = sizeof(T) == 4 && el.nv % 4 == 0 && (reinterpret_cast<uintptr_t>(ul) & 15u) == 0 &&
+    auto add = [&](T fac, T a, T b) {
+        if (fac >= T(0)) s0 += double(fac * a);
+        else s1 += double(fac * b);
+    };
+    // four velocities of one z line per step (16-byte loads) when rows are
+    // aligned and 4 divides Nv
+    const bool v4 = Nv % 4 == 0 && (reinterpret_cast<uintptr_t>(ul) & 15u) == 0 &&
                     (reinterpret_cast<uintptr_t>(fw) & 15u) == 0;
-    const bool zline = el.Nv % 4 == 0;
-    const int64_t nv4 = v4 ? el.nv : 0;
-    for (int64_t v0 = int64_t(threadIdx.x) * 4; v0 < nv4; v0 += int64_t(blockDim.x) * 4) {
-        Vec<T, 4> a, b;
-        a.load(ul + v0);
-        b.load(fw + v0);
-        const uint32_t vv = uint32_t(v0), nn = uint32_t(el.Nv);    // v < Nv^3 <= 2^30
-        const uint32_t qq = vv / nn, iz0 = vv - qq * nn;
-        const uint32_t ix = qq / nn, iy = qq - ix * nn;
+    if (v4) {
+        const uint32_t n = uint32_t(el.nv), st = blockDim.x * 4;
+        RowWalk x(threadIdx.x * 4, st, uint32_t(Nv));
+        auto step = [&](const Chunk<T, 4>& a, const Chunk<T, 4>& b) {
+            const T f0 = (cs[x.ix] - uw[0]) * pn[0], f1 = (cs[x.iy] - uw[1]) * pn[1];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            T c[3];
-            if (zline) {
-                c[0] = cs[ix];
-                c[1] = cs[iy];
-                c[2] = cs[iz0 + q];
-            } else {
-                vel(cs, el.Nv, v0 + q, c);
+            for (int q = 0; q < 4; ++q) add(f0 + f1 + (cs[x.iz + q] - uw[2]) * pn[2], a.v[q], b.v[q]);
+            x.next();
+        };
+        for (uint32_t v = threadIdx.x * 4; v < n; v += 2 * st) {
+            Chunk<T, 4> a[2], b[2];
+            a[0].load(ul + v);
+            b[0].load(fw + v);
+            const bool two = v + st < n;
+            if (two) {
+                a[1].load(ul + v + st);
+                b[1].load(fw + v + st);
             }
-            T fac = T(0);
-            for (int d = 0; d < ND; ++d) fac += (c[d] - uw[d]) * pn[d];
-            if (fac >= T(0)) s0 += double(fac * a.v[q]);
-            else s1 += double(fac * b.v[q]);
+            step(a[0], b[0]);
+            if (two) step(a[1], b[1]);
         }
-    }
-    for (int64_t v = nv4 + threadIdx.x; v < el.nv; v += blockDim.x) {
-        T c[3];
-        vel(cs, el.Nv, v, c);
-        T fac = T(0);
-        for (int d = 0; d < ND; ++d) fac += (c[d] - uw[d]) * pn[d];
-        if (fac >= T(0)) s0 += double(fac * ul[v]);
-        else s1 += double(fac * fw[v]);
+    } else {
+        for (int64_t v = threadIdx.x; v < el.nv; v += blockDim.x) {
+            T c[3];
+            vel(cs, Nv, v, c);
+            add((c[0] - uw[0]) * pn[0] + (c[1] - uw[1]) * pn[1] + (c[2] - uw[2]) * pn[2], ul[v], fw[v]);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         s0 += __shfl_xor_sync(0xffffffffu, s0, o);
@@ -682,6 +631,9 @@ __global__ void __launch_bounds__(256) bc_update_kernel(const bdgfs_fr_eles el,
         out[2 * w + 1] = T(a1 * wl.cw);
     }
 }
+
+// threads per wall point: 1024 while two such CTAs per SM hold every point
+static unsigned bc_update_threads(int nwall) { return nwall <= 148 * 2 ? 1024 : nwall <= 148 * 4 ? 512 : 256; }
 
 template <typename T>
 __global__ void __launch_bounds__(256) residual_kernel(const T* __restrict__ a,
@@ -746,17 +698,6 @@ static int grid_v(int64_t nv, int neles, int64_t chunk, dim3* g)
     if (bx > 65535 || neles > 65535 || neles < 1) return BDGFS_EINVAL;
     *g = dim3(unsigned(bx), unsigned(neles));
     return BDGFS_OK;
-}
-
-// VB velocities per thread when every row is VB-aligned
-template <typename T>
-static int vec_width(int64_t nv, const void* const* ptrs, int n)
-{
-    const int VB = sizeof(T) == 4 ? 4 : 2;
-    if (nv % VB) return 1;
-    for (int i = 0; i < n; ++i)
-        if (ptrs[i] && (reinterpret_cast<uintptr_t>(ptrs[i]) % (VB * sizeof(T)))) return 1;
-    return VB;
 }
 
 template <typename T, int ND, int NU, int NF, int VB, int TPP = 0>
@@ -893,10 +834,10 @@ extern "C" int32_t bdgfs_fr_bc_update(const bdgfs_fr_eles* el, const bdgfs_fr_wa
         return BDGFS_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (el->fp64)
-        bc_update_kernel<double><<<wl->nwall, 256, 0, st>>>(*el, *wl, static_cast<const double*>(uf),
+        bc_update_kernel<double><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const double*>(uf),
                                                             nullptr);
     else
-        bc_update_kernel<float><<<wl->nwall, 256, 0, st>>>(*el, *wl, static_cast<const float*>(uf),
+        bc_update_kernel<float><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const float*>(uf),
                                                            nullptr);
     return cuda_status(cudaGetLastError());
 }
@@ -912,9 +853,9 @@ extern "C" int32_t bdgfs_fr_bc_update_gather(const bdgfs_fr_eles* el, const bdgf
         return BDGFS_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (el->fp64)
-        bc_update_kernel<double><<<wl->nwall, 256, 0, st>>>(*el, *wl, static_cast<const double*>(u), fsel);
+        bc_update_kernel<double><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const double*>(u), fsel);
     else
-        bc_update_kernel<float><<<wl->nwall, 256, 0, st>>>(*el, *wl, static_cast<const float*>(u), fsel);
+        bc_update_kernel<float><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const float*>(u), fsel);
     return cuda_status(cudaGetLastError());
 }
 
