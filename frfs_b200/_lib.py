@@ -19,7 +19,7 @@ EXPORTS = (
     'bdgfs_vhs_scratch_bytes', 'bdgfs_vhs_collide', 'bdgfs_vhs_tiles', 'bdgfs_fma_probe',
     'bdgfs_vhs_collide_static', 'bdgfs_wait_probe',
     'bdgfs_fr_disu', 'bdgfs_fr_invmass', 'bdgfs_fr_bc_update', 'bdgfs_fr_rhs', 'bdgfs_fr_rhs_gather',
-    'bdgfs_fr_bc_update_gather', 'bdgfs_fr_rhs_tensor',
+    'bdgfs_fr_bc_update_gather', 'bdgfs_fr_rhs_tensor', 'bdgfs_fr_rhs_affine',
     'bdgfs_moments', 'bdgfs_macroscopic', 'bdgfs_residual', 'bdgfs_status_check',
     'bdgfs_gemm', 'bdgfs_colsum', 'bdgfs_adamw', 'bdgfs_relmse',
     'bdgfs_hybrid_classify', 'bdgfs_hybrid_project', 'bdgfs_hybrid_scatter',
@@ -73,6 +73,12 @@ class FrWall(C.Structure):
 
 
 BC_DIFFUSE, BC_INLET, BC_OUTLET, BC_SPECULAR_X, BC_SPECULAR_Y, BC_SPECULAR_Z = range(6)
+
+
+class FrAffine(C.Structure):
+    _fields_ = [('fsel', C.c_void_p), ('fid', C.c_void_p), ('smat', C.c_void_p),
+                ('d', C.c_double * 16), ('kw', C.c_double * 16), ('kn', C.c_double * 8),
+                ('p', C.c_int32), ('pad_', C.c_int32)]
 
 
 class GemmArgs(C.Structure):
@@ -179,6 +185,7 @@ def lib():
             'bdgfs_fr_bc_update_gather': [vp, vp, vp, vp, vp],
             'bdgfs_fr_rhs_tensor': [vp, vp, vp, vp, vp, vp, dbl, dbl, vp, dbl, vp, dbl, vp],
             'bdgfs_moments': [vp, i64, i32, i32, vp, dbl, vp, vp],
+            'bdgfs_fr_rhs_affine': [vp, vp, vp, vp, vp, vp, dbl, dbl, vp, dbl, vp, dbl, vp],
             'bdgfs_macroscopic': [vp, i64, i32, i32, vp, dbl, vp, vp, vp, vp, vp, vp],
             'bdgfs_residual': [vp, vp, i64, i32, vp, vp],
             'bdgfs_status_check': [vp, i64, i32, vp, vp],

@@ -46,6 +46,7 @@ class DGFSElements:
         unit = np.all(np.count_nonzero(m0, axis=1) == 1) and np.all(m0.max(axis=1) == 1.0)
         self.fsel = (backend.const(np.argmax(m0, axis=1), dtype=torch.int32) if unit else None)
         self.tensor = self._tensor_form(shp, m0, c) if unit else None
+        self.affine = self._affine_form(shp, m0) if self.tensor is not None else None
         self.dcorr = c(shp.opmat('M1 - M3*M2'))
         self.m3 = c(shp.opmat('M3'))
         self.minv = c(shp.opmat('M12'))
@@ -98,6 +99,64 @@ class DGFSElements:
         self.tp_fsel = self.be.const(fsel, dtype=torch.int32)
         return _lib.FrTensor(fsel=self.tp_fsel.data_ptr(), fdim=self.tp_fdim.data_ptr(),
                              fsgn=self.tp_fsgn.data_ptr(), m1line=self.tp_m1line.data_ptr(), p=p)
+
+    def _affine_form(self, shp, m0):
+        """bdgfs_fr_affine of the elements when their metric is one matrix each
+        (the face normals are its rows then) and M3 factors along the axes;
+        else None."""
+        geo, nd, nu, nf = self.geo, self.ndims, self.nupts, self.nfpts
+        p = shp.n1
+        S, nref = np.asarray(geo.smats, np.float64), np.asarray(shp.norm_fpts)
+        if np.any(S != S[:, :1]) or np.any(geo.rcpdjac != np.asarray(geo.rcpdjac)[:, :1]):
+            return None
+        S = S[:, 0]                                              # [E][ND][ND]
+        pn = np.asarray(geo.norm_pnorm) * np.asarray(geo.mag_pnorm)[..., None]
+        if not np.allclose(pn, np.einsum('fi,eik->efk', nref, S), rtol=1e-12,
+                           atol=1e-13 * np.abs(pn).max()):
+            return None
+        m1, m3, fsel = np.asarray(shp.opmat('M1')), np.asarray(shp.opmat('M3')), np.argmax(m0, axis=1)
+        st = [p**d for d in range(nd)]
+        D = np.array([[m1[i * st[0], j * st[0]] for j in range(p)] for i in range(p)])
+        fid = np.zeros((2 * nd, p**(nd - 1)), dtype=np.int32)
+        for f in range(nf):
+            d = int(np.argmax(np.abs(nref[f])))
+            idx = [(fsel[f] // st[a]) % p for a in range(nd) if a != d]
+            side = int(nref[f, d] > 0)
+            if idx and (fsel[f] // st[d]) % p != side * (p - 1):
+                return None
+            fid[2 * d + side, sum(i * p**k for k, i in enumerate(idx))] = f
+        # M3[(u), f] = kn[side][u_d] prod kw[u_t][f_t]: read kn off at matching
+        # tangential points and kw off relative to them, then check every entry
+        f0 = [fid[2 * 0 + s, 0] for s in (0, 1)]
+        ref = m3[0, f0[0]]
+        if ref == 0.0:
+            return None
+        kt = np.array([[m3[i * st[1], fid[0, j]] for j in range(p)] for i in range(p)])
+        kw = kt / kt[0, 0] if nd == 2 else None
+        if nd == 3:
+            kt = np.array([[m3[i * st[1], fid[0, j]] for j in range(p)] for i in range(p)])
+            kw = kt / kt[0, 0]
+        # scale so that kw is the factor itself (rows of K w sum like a quadrature
+        # of the constant: sum_j kw[i][j] = 1)
+        kw = kw / kw[0].sum()
+        kn = np.array([[m3[i * st[0], f0[s]] for i in range(p)] for s in (0, 1)]) / kw[0, 0]**(nd - 1)
+        for f in range(nf):
+            d, side = int(np.argmax(np.abs(nref[f]))), int(nref[f].sum() > 0)
+            col = np.ones(nu)
+            for a in range(nd):
+                ua = (np.arange(nu) // st[a]) % p
+                col *= kn[side][ua] if a == d else kw[ua, (fsel[f] // st[a]) % p]
+            if not np.allclose(col, m3[:, f], rtol=0, atol=1e-12 * np.abs(m3).max()):
+                return None
+        self.af_fid = self.be.const(fid, dtype=torch.int32)
+        self.af_smat = self.be.const(np.ascontiguousarray(S), dtype=self.be.fpdtype)
+        a = _lib.FrAffine(fsel=self.fsel.data_ptr(), fid=self.af_fid.data_ptr(),
+                          smat=self.af_smat.data_ptr(), p=p)
+        for i in range(p):
+            for j in range(p):
+                a.d[i * p + j], a.kw[i * p + j] = D[i, j], kw[i, j]
+            a.kn[i], a.kn[p + i] = kn[0, i], kn[1, i]
+        return a
 
     def ploc_at_np(self, name):
         return {'upts': self.geo.plocupts, 'fpts': self.geo.plocfpts}[name]
@@ -383,6 +442,12 @@ class DGFSSystem:
         L = _lib.lib()
         xs = (float(a), float(b), x1.data_ptr() if x1 is not None else None, float(c1),
               x2.data_ptr() if x2 is not None else None, float(c2), _lib.stream_ptr())
+        if self.ele.tensor is not None and self.ele.affine is not None and self.ele.struct.engine == 0:
+            rc = L.bdgfs_fr_rhs_affine(_lib.ref(self.ele.struct), _lib.ref(self.walls.struct),
+                                       _lib.ref(self.ele.affine), u.data_ptr(),
+                                       self._uf_rows.data_ptr(), out.data_ptr(), *xs)
+            _lib.check(rc, 'bdgfs_fr_rhs_affine')
+            return
         if self.ele.tensor is not None and self.ele.struct.engine == 0:
             rc = L.bdgfs_fr_rhs_tensor(_lib.ref(self.ele.struct), _lib.ref(self.walls.struct),
                                        _lib.ref(self.ele.tensor), u.data_ptr(),
@@ -462,7 +527,13 @@ class DGFSSystem:
                            'bdgfs_fr_bc_update_gather')
             xs = (x1.data_ptr() if x1 is not None else None, float(c1),
                   x2.data_ptr() if x2 is not None else None, float(c2), _lib.stream_ptr())
-            if self.ele.tensor is not None:
+            if self.ele.tensor is not None and self.ele.affine is not None:
+                _lib.check(L.bdgfs_fr_rhs_affine(_lib.ref(self.ele.struct),
+                                                 _lib.ref(self.walls.struct),
+                                                 _lib.ref(self.ele.affine), u.data_ptr(), None,
+                                                 out.data_ptr(), float(a), float(b), *xs),
+                           'bdgfs_fr_rhs_affine')
+            elif self.ele.tensor is not None:
                 _lib.check(L.bdgfs_fr_rhs_tensor(_lib.ref(self.ele.struct),
                                                  _lib.ref(self.walls.struct),
                                                  _lib.ref(self.ele.tensor), u.data_ptr(), None,

@@ -259,6 +259,32 @@ int32_t bdgfs_fr_rhs_tensor(const bdgfs_fr_eles* el, const bdgfs_fr_walls* wl,
                             const void* x1, double c1, const void* x2,
                             double c2, void* stream);
 
+/* Affine elements (one metric matrix per element) of a tensor-product shape
+ * with flux points on solution points: the same residual from 1-D factors,
+ * with only the inflow face of each direction read (the outflow face's
+ * F^n - M2 F~ is zero). */
+typedef struct bdgfs_fr_affine {
+    const int32_t* fsel;  /* [nfpts] solution point of flux point f           */
+    const int32_t* fid;   /* [2 ndims][p^(ndims-1)] flux point of the lower
+                             (2d) and upper (2d+1) face of direction d at
+                             tangential point t (first remaining axis fastest) */
+    const void* smat;     /* real [neles][ndims][ndims]: smats of the element */
+    double d[16];         /* [p][p] 1-D derivative: (D u)_i = sum_j d[i][j] u_j */
+    double kw[16];        /* [p][p] tangential factor of M3 on a face axis    */
+    double kn[8];         /* [2][p] normal factor of M3, lower and upper face */
+    int32_t p;            /* points per line, 2..4                            */
+    int32_t pad_;
+} bdgfs_fr_affine;
+
+/* bdgfs_fr_rhs_tensor (uf = the face values; or NULL, out must not alias u
+ * then) for affine elements, equal to rounding, and bitwise the same with or
+ * without uf.  Reads el's rcpdjac (the element's first), nbr and c0. */
+int32_t bdgfs_fr_rhs_affine(const bdgfs_fr_eles* el, const bdgfs_fr_walls* wl,
+                            const bdgfs_fr_affine* af, const void* u,
+                            const void* uf, void* out, double a, double b,
+                            const void* x1, double c1, const void* x2,
+                            double c2, void* stream);
+
 /* FP64 raw velocity moments of ndof distributions, out[ndof][13]:
  * cw*sum{f, c f (3), c_i c_j f (xx xy xz yy yz zz), |c|^2 c f (3)}.
  * Feeds the macroscopic fields of plugins/dgfsmomwriterstd.py:14-313. */
