@@ -115,15 +115,26 @@ class VHSGrid:
             ginv=self.ginv.data_ptr())
 
 
+# tile value of a grid set that ``autotune.tune_vhs`` found faster as one launch
+# per grid (no tile index of bdgfs_vhs_tiles)
+BY_GRID = -1
+
+
 class VHSCollider:
     """Owns scratch and the work counter for one set of grids and runs
-    ``bdgfs_vhs_collide`` (one persistent launch over all batches)."""
+    ``bdgfs_vhs_collide`` (one persistent launch over all batches; with tile
+    BY_GRID one launch per grid, each on its own tuned tile)."""
 
     def __init__(self, grids, device):
         self.grids = list(grids)
         self.device = device
         if any(g.phase.device.type != 'cuda' for g in self.grids):
             raise _lib.BdgfsError('collision tables must be on a CUDA device')
+        self._each = None
+        if self.grids[0].struct.tile == BY_GRID:
+            from .autotune import tuned_alone
+            self._each = [VHSCollider([tuned_alone(g, device)], device) for g in self.grids]
+            return
         arr = (_lib.VhsGrid * len(self.grids))(*[g.struct for g in self.grids])
         self._garr = arr
         L = _lib.lib()
@@ -137,6 +148,13 @@ class VHSCollider:
         """batches: list of (grid_index, f[ndof, n], Q[ndof, n], moments|None).
         index (int32, device) / count (int64 device scalar) restrict the first
         batch to f[index[i]], i < count (read by the kernel)."""
+        if self._each is not None:
+            for gi, col in enumerate(self._each):
+                own = [(0,) + tuple(b[1:]) for b in batches if b[0] == gi]
+                if own:
+                    first = batches[0][0] == gi
+                    col(own, project, exact, stream, index if first else None, count if first else None)
+            return
         L = _lib.lib()
         bs = (_lib.VhsBatch * len(batches))()
         for i, (gi, f, Q, mom) in enumerate(batches):
