@@ -1,29 +1,59 @@
 // Cutting the work of a few long items into parts.
+//
+// An item is ``nb`` equal blocks of work (radii) whose results are rounded and then
+// added in order, by its one CTA or, if cut, from a slot per block by the part that
+// ends last: an item's result has the same bits whole or cut, wherever it stands
+// in a list and however many CTAs run.
 #pragma once
 #include <cstdint>
 
 namespace bdgfs {
 
-constexpr int kMaxParts = 16;
+// Items [0, whole) are done whole, the others in ``ns`` parts each.
+struct SplitPlan {
+    int64_t whole;
+    int ns;
+};
 
-// Parts that each of ``total`` items of ``units`` equal units is cut into on
-// ``ncta`` CTAs: the number with the smallest (rounds of CTAs) x (units per part
-// + what every part repeats, in units: ``once`` uncut, ``again`` for a part), so
-// that a few items occupy the SMs and a nearly empty last round costs a part of
-// an item's time only.  Cutting needs a slot per part.
-__host__ __device__ inline int split_parts(int64_t total, int64_t nslots, int units, int ncta, float once, float again)
+// Plan for ``total`` items of ``nb`` blocks on ``ncta`` CTAs: full rounds of CTAs are
+// left whole; the items of the last, partly filled round (or of a list shorter
+// than the CTAs) are cut into the number of parts with the smallest (rounds of
+// CTAs) x (blocks per part + what every part repeats, in blocks: ``once`` uncut,
+// ``again`` for a part).  A cut item needs ``nb`` of ``nslots`` slots.
+__host__ __device__ inline SplitPlan split_plan(int64_t total, int64_t nslots, int nb, int ncta, float once, float again)
 {
+    const int64_t tail = total % ncta;
     int best = 1;
     float cost = 1e30f;
-    for (int ns = 1; ns <= (units < kMaxParts ? units : kMaxParts); ++ns) {
-        if (ns > 1 && total * ns > nslots) break;
-        const float c = float((total * ns + ncta - 1) / ncta) * (float((units + ns - 1) / ns) + (ns > 1 ? again : once));
+    for (int ns = 1; tail > 0 && ns <= nb; ++ns) {
+        if (ns > 1 && tail * nb > nslots) break;
+        const float c = float((tail * ns + ncta - 1) / ncta) * (float((nb + ns - 1) / ns) + (ns > 1 ? again : once));
         if (c < 0.97f * cost) {
             cost = c;
             best = ns;
         }
     }
-    return best;
+    return SplitPlan{best > 1 ? total - tail : total, best};
+}
+
+// Work item -> position in the list, its blocks [b0, b1) of nb, parts of it, and
+// its place among the cut items
+struct SplitItem {
+    int64_t li, cut;
+    int b0, b1, ns;
+};
+
+__device__ __forceinline__ SplitItem split_item(int64_t item, const SplitPlan& p, int nb)
+{
+    if (item < p.whole) return SplitItem{item, 0, 0, nb, 1};
+    const int64_t k = item - p.whole, cut = k / p.ns;
+    const int part = int(k - cut * p.ns);
+    return SplitItem{p.whole + cut, cut, nb * part / p.ns, nb * (part + 1) / p.ns, p.ns};
+}
+
+__host__ __device__ inline int64_t split_items(int64_t total, const SplitPlan& p)
+{
+    return p.whole + (total - p.whole) * p.ns;
 }
 
 }  // namespace bdgfs

@@ -1579,18 +1579,15 @@ static int launch(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch
     return cuda_status(cudaGetLastError());
 }
 
-// The shift-tree kernel.  The exact-Nyquist mode (BDGFS_EXACT) has a second
-// transform per direction that does not factor; it runs on the
-// spectra-in-TMEM variant.  Scratch: tickets and slots of partial gains for
-// distributions split over radii (tree_split), as many as fit.
-static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
-                       int nbatch, int flags, void* scratch, size_t scratch_bytes,
-                       uint64_t* counter, cudaStream_t st)
+// Arguments and grid of a kernel that cuts short lists over radii: the scratch
+// holds tickets, and per CTA ``priv`` bytes and a slot (G^), then as many slots for
+// the radii of cut distributions as fit; the plan is made in the kernel (a batch's
+// count may be on the device), and here for the grid.  Clears the counter and the tickets; *nblk = 0: nothing to do.
+template <typename Args>
+static int split_launch(Args& a, const bdgfs_vhs_grid* grids, const bdgfs_vhs_batch* batches, int nbatch, int flags,
+                        void* scratch, size_t scratch_bytes, uint64_t* counter, size_t priv, size_t slot, int ctas_per_sm,
+                        float once, float again, cudaStream_t st, int64_t* nblk, unsigned char** private_at)
 {
-    if (flags & BDGFS_EXACT)
-        return launch<float, 320, VariantP2<true, true, true>, NoVariant>(
-            grids, ngrids, batches, nbatch, flags, scratch, scratch_bytes, counter, st);
-    TreeArgs a{};
     a.g = grids[0];
     a.nbatch = nbatch;
     a.flags = flags;
@@ -1602,29 +1599,54 @@ static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_
         total += batches[b].ndof;
         dev_count = dev_count || batches[b].count;
     }
+    *nblk = 0;
     if (total == 0) return BDGFS_OK;
-    if (scratch_bytes < QLayoutP2::scratch_bytes()) return BDGFS_ESCRATCH;
     int dev = 0, nsm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return BDGFS_ECUDA;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return BDGFS_ECUDA;
     const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
     const size_t room = scratch_bytes - std::min(scratch_bytes, size_t(base - reinterpret_cast<uintptr_t>(scratch)));
-    const int64_t fit = int64_t(room / (QLayoutTree::slot_bytes() + 256));
-    if (fit < 1) return BDGFS_ESCRATCH;
+    const int64_t ctas = std::min<int64_t>(int64_t(nsm) * ctas_per_sm, int64_t(room / (priv + slot + 256)));
+    if (ctas < 1) return BDGFS_ESCRATCH;
+    // tickets, private parts, a slot per CTA, slots of cut distributions
+    const size_t head = (size_t(ctas) * sizeof(uint32_t) + 255) / 256 * 256, used = head + size_t(ctas) * (priv + slot);
+    a.nctas = int32_t(ctas);
     a.tickets = reinterpret_cast<uint32_t*>(base);
-    a.slots = reinterpret_cast<unsigned char*>(base + (size_t(fit) * sizeof(uint32_t) + 255) / 256 * 256);
-    int64_t parts = std::min(a.g.Nrho, kMaxParts);
-    if (!dev_count) parts = tree_split(total, fit, a.g.Nrho, nsm);
-    if (parts > 1) {
-        a.nslots = fit;
-        if (cudaMemsetAsync(a.tickets, 0, size_t(std::min(total, fit)) * sizeof(uint32_t), st) != cudaSuccess)
-            return BDGFS_ECUDA;
-    }
-    const int64_t nblk = std::min(std::min<int64_t>(nsm, fit), total * parts);
+    unsigned char* at = reinterpret_cast<unsigned char*>(base + head);
+    a.slots = at + size_t(ctas) * priv;
+    *private_at = at;
+    a.nslots = room > used ? int64_t((room - used) / slot) : 0;
+    SplitPlan plan{total, 1};
+    if (!dev_count) plan = split_plan(total, a.nslots, a.g.Nrho, int(ctas), once, again);
+    const int64_t cut = dev_count ? std::min(total, ctas) : total - plan.whole;     // one ticket each
+    if (cut > 0 && cudaMemsetAsync(a.tickets, 0, size_t(cut) * sizeof(uint32_t), st) != cudaSuccess)
+        return BDGFS_ECUDA;
+    if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), st) != cudaSuccess) return BDGFS_ECUDA;
+    *nblk = std::min(ctas, dev_count ? total * a.g.Nrho : split_items(total, plan));
+    return BDGFS_OK;
+}
+
+// The shift-tree kernel.  The exact-Nyquist mode (BDGFS_EXACT) has a second
+// transform per direction that does not factor; it runs on the
+// spectra-in-TMEM variant.
+static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                       int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                       uint64_t* counter, cudaStream_t st)
+{
+    if (flags & BDGFS_EXACT)
+        return launch<float, 320, VariantP2<true, true, true>, NoVariant>(
+            grids, ngrids, batches, nbatch, flags, scratch, scratch_bytes, counter, st);
+    if (scratch_bytes < QLayoutP2::scratch_bytes()) return BDGFS_ESCRATCH;
+    TreeArgs a{};
+    int64_t nblk = 0;
+    unsigned char* none = nullptr;
+    if (const int rc = split_launch(a, grids, batches, nbatch, flags, scratch, scratch_bytes, counter, 0,
+                                    QLayoutTree::slot_bytes(), 1, 1.5f, 1.7f, st, &nblk, &none))
+        return rc;
+    if (nblk == 0) return BDGFS_OK;
     const size_t smem = QLayoutTree::smem_bytes(a.g.M);
     if (const int rc = smem_optin(reinterpret_cast<const void*>(vhs_tree_kernel), smem)) return rc;
-    if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), st) != cudaSuccess) return BDGFS_ECUDA;
     vhs_tree_kernel<<<unsigned(nblk), tree::NT, smem, st>>>(a);
     return cuda_status(cudaGetLastError());
 }

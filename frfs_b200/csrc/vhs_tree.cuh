@@ -32,17 +32,18 @@
 // Work per radius at 12 directions: 2 + 6 passes of 312 pencil pairs and one of
 // 6 x 576, against 36 passes of 288 pairs, and 8 exchanges of a 120 KB cube
 // through shared memory against 24 of 110 KB.  Measured on one B200, Nrho = 12,
-// 12 directions: 2048 distributions 9.79 -> 6.17 ms (the variant with spectra
-// in tensor memory -> this one), 97 0.703 -> 0.349 ms, one 0.699 -> 0.087 ms
-// (radii split over CTAs); the error against 64-bit arithmetic falls from
-// 4.5e-5 to 1e-5 of Q (fewer roundings into S_p).  Bound: the FP32 pipe (48 %
+// 12 directions: 2048 distributions 9.79 -> 6.09 ms (the variant with spectra
+// in tensor memory -> this one), 97 0.705 -> 0.358 ms, one 0.706 -> 0.085 ms
+// (radii cut over CTAs, split.cuh; so is the last, partly filled round of a long
+// list: 6.17 -> 6.09 ms for the 2048); the error against 64-bit arithmetic falls
+// from 4.5e-5 to 1e-5 of Q (fewer roundings into S_p).  Bound: the FP32 pipe (48 %
 // busy, 57 % on the sub-partitions with three warps) and the barriers of the
 // exchanges (shared memory 40 %).
 //
 // One CTA of 320 threads per distribution.  Thread t < 312 owns the pencil
 // (i, kz) = (t % 24, t / 24): ky in the x-passes, x in the y-passes.  Leaves:
-// thread t owns the z-pencils t and t + 320 (of 576, x fastest).  Exchange elements are (A.re, B.re, A.im, B.im): one 16-byte
-// access each, free of bank conflicts (row pitch 313 where the pencil axis
+// thread t owns the z-pencils t and t + 320 (of 576, x fastest).  Exchange
+// elements are (A.re, B.re, A.im, B.im): one 16-byte access each, free of bank conflicts (row pitch 313 where the pencil axis
 // changes, 312 else).  F lives in shared memory; the x-node's pencils and S_p in
 // tensor memory, where only their own thread reads them (10 warps put three on
 // two of the SM's sub-partitions, which caps registers at 168); the spectral
@@ -86,8 +87,9 @@ struct QLayoutTree {
     }
     // G^ of one CTA, or of one work item when distributions are split over radii
     static constexpr size_t slot_bytes() { return size_t(tree::N) * tree::NT * sizeof(float2); }
-    // per CTA: 4 slots and tickets
-    static size_t scratch_bytes() { return 4 * (slot_bytes() + 256); }
+    // per CTA: its slot, and eight for the radii of cut distributions
+    static constexpr int kCut = 8;
+    static size_t scratch_bytes() { return (1 + kCut) * (slot_bytes() + 256); }
 };
 
 struct TreeArgs {
@@ -95,8 +97,9 @@ struct TreeArgs {
     bdgfs_vhs_batch batches[4];
     int32_t nbatch, flags;
     unsigned char* slots;
-    uint32_t* tickets;              // one per distribution, zeroed before the launch (split launches)
-    int64_t nslots;                 // 0: no splitting (one slot per CTA)
+    uint32_t* tickets;              // one per cut distribution, zeroed before the launch
+    int64_t nslots;                 // slots of cut distributions' radii, after one per CTA
+    int32_t nctas;                  // CTAs that a full round has
     unsigned long long* counter;
 };
 
@@ -152,21 +155,14 @@ __device__ inline void tree_plan(const cpx<float>* phase, int Nrho, int M, TreeP
     }
 }
 
-// Parts that each distribution's radii are cut into (split.cuh); F and the final
-// transforms cost about 1.5 radii, the sum of the parts 0.2 more.  97
-// distributions on 148 SMs: 3 parts, 0.349 ms against 0.44 ms uncut.
-__host__ __device__ inline int tree_split(int64_t total, int64_t nslots, int Nrho, int ncta)
-{
-    return split_parts(total, nslots, Nrho, ncta, 1.5f, 1.7f);
-}
-
 __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
 {
     using namespace tree;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int64_t s_item;
     __shared__ int64_t s_start[5];
-    __shared__ int s_split, s_last;
+    __shared__ SplitPlan s_plan;
+    __shared__ int s_last;
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_free;
     __shared__ TreePlan pl;
@@ -205,7 +201,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
             }
             s_start[b + 1] = s_start[b] + c;
         }
-        s_split = tree_split(s_start[a.nbatch], a.nslots, Nrho, int(gridDim.x));
+        s_plan = split_plan(s_start[a.nbatch], a.nslots, Nrho, a.nctas, 1.5f, 1.7f);
     }
     __syncthreads();
     tc::tc_fence_after();
@@ -314,16 +310,17 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
     };
 
     const int64_t total = s_start[a.nbatch];
-    const int ns = s_split;
-    const int64_t nitems = total * ns;
+    const SplitPlan plan = s_plan;
+    const int64_t nitems = split_items(total, plan);
     for (;;) {
         if (tid == 0) s_item = int64_t(atomicAdd(a.counter, 1ull));
         __syncthreads();
         const int64_t item = s_item;
         __syncthreads();
         if (item >= nitems) break;
-        const int64_t li = item / ns;
-        const int part = int(item - li * ns);
+        const SplitItem it = split_item(item, plan, Nrho);
+        const int64_t li = it.li;
+        const int ns = it.ns;
         int b = 0;
         while (li >= s_start[b + 1]) ++b;
         const bdgfs_vhs_batch& bt = a.batches[b];
@@ -351,10 +348,10 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
             }
         }
 
-        float2* G = reinterpret_cast<float2*>(a.slots + size_t(ns > 1 ? item : int64_t(blockIdx.x)) *
-                                              QLayoutTree::slot_bytes()) + tid;    // [kx * NT]
-        const int p0 = Nrho * part / ns, p1 = Nrho * (part + 1) / ns;
-        for (int p = p0; p < p1; ++p) {
+        // G^ of this thread, [kx * NT]: the sum so far, or one slot per radius (cut)
+        const int64_t slot = ns > 1 ? a.nctas + it.cut * Nrho + it.b0 : int64_t(blockIdx.x);
+        float2* G = reinterpret_cast<float2*>(a.slots + size_t(slot) * QLayoutTree::slot_bytes()) + tid;
+        for (int p = it.b0; p < it.b1; ++p) {
             // ---- node factors of radius p ----
             const cpx<float>* php = phase + size_t(p) * M * 3 * N;
             for (int i = tid; i < (pl.nx + pl.ny) * N; i += NT) {
@@ -545,35 +542,37 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
                 cpx<float> X[N];
                 forward(u0, u1, X);
                 const float* gwp = gw + (size_t(p) * N + kz) * HP * N + pi;
+                const bool acc = ns == 1 && p > 0;
 #pragma unroll
                 for (int kx = 0; kx < N; ++kx) {
                     const float w = ldg(gwp + (kx <= H ? kx : N - kx) * N);
-                    const float2 o = p > p0 ? G[kx * NT] : f2(0.f, 0.f);
-                    G[kx * NT] = f2(fmaf(w, X[kx].x, o.x), fmaf(w, X[kx].y, o.y));
+                    const float2 o = acc ? G[kx * NT] : f2(0.f, 0.f);
+                    G[kx * NT] = f2(__fadd_rn(o.x, __fmul_rn(w, X[kx].x)), __fadd_rn(o.y, __fmul_rn(w, X[kx].y)));
                 }
+                if (ns > 1) G += N * NT;
             }
         }
 
         float2 vr[N], vi[N];                              // lane A: this thread's G^
         if (ns > 1) {
-            // the part that arrives last adds the parts' gains in order and
-            // finishes the distribution
+            // the part that arrives last adds the radii in order and finishes the
+            // distribution
             __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(a.tickets + li, 1u) == uint32_t(ns - 1);
+            if (tid == 0) s_last = atomicAdd(a.tickets + it.cut, 1u) == uint32_t(ns - 1);
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
-            const float2* Gj = reinterpret_cast<const float2*>(a.slots + size_t(li) * ns * QLayoutTree::slot_bytes()) + tid;
+            const float2* Gj = reinterpret_cast<const float2*>(a.slots + size_t(a.nctas + it.cut * Nrho) * QLayoutTree::slot_bytes()) + tid;
 #pragma unroll
             for (int k = 0; k < N; ++k) vr[k].x = vi[k].x = 0.f;
 #pragma unroll 1
-            for (int j = 0; j < ns; ++j, Gj += N * NT) {
+            for (int j = 0; j < Nrho; ++j, Gj += N * NT) {
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
                     const float2 v = __ldcg(Gj + k * NT);
-                    vr[k].x += v.x;
-                    vi[k].x += v.y;
+                    vr[k].x = __fadd_rn(vr[k].x, v.x);
+                    vi[k].x = __fadd_rn(vi[k].x, v.y);
                 }
             }
         } else {

@@ -19,8 +19,9 @@
 // group of eight rows.  G^ of both species stays in tensor memory.  F comes from
 // the CTA's scratch and the weights from their tables, through L2: 165 KB (like
 // pair) or 442 KB a slice.  Measured on one B200, Nrho = M = 12, 370 argon-krypton
-// pairs: 25.5 -> 12.2 ms (the general kernel of vss.cu -> this one); error against
-// 64-bit arithmetic 4.2e-6 -> 4.9e-6 of Q.  Bound: the FP32 pipe and the barriers
+// pairs: 25.6 -> 10.9 ms (the general kernel of vss.cu -> this one; 12.3 ms before
+// the last round's distributions were cut over radii); error against 64-bit
+// arithmetic 4.0e-6 -> 3.5e-6 of Q.  Bound: the FP32 pipe and the barriers
 // between passes.  (The factors are real but for Nyquist terms; packing them as
 // one complex transform drops those terms, 1e-3 of Q on this mixture.)
 #include <algorithm>
@@ -45,14 +46,49 @@ constexpr size_t kSlot = size_t(N) * NZ * sizeof(float4);    // partial G^ of bo
 struct VssPairArgs {
     bdgfs_vss_pair_args g;
     unsigned char* F;                // [CTA] kF
-    unsigned char* slots;            // [item] kSlot (split launches)
-    uint32_t* tickets;               // [distribution], zeroed (split launches)
-    int32_t ns;                      // parts per distribution
+    unsigned char* sums;             // [CTA] kSlot: sum of the radii
+    unsigned char* slots;            // [cut distribution][radius] kSlot
+    uint32_t* tickets;               // [cut distribution], zeroed
+    SplitPlan plan;
     uint32_t* timeout;               // set when a bounded wait ran out
 };
 
 __device__ __forceinline__ float2 v2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+
+// The thread's accumulators (ntask pencils in tensor memory) to zero, and out to
+// ``to`` [kx][NZ], added to what it holds if ``add``.  Once per radius: calls, so that
+// their registers do not count in the slices' loop.
+__device__ __noinline__ void vssp_clear(uint32_t tcol, int ntask)
+{
+    uint32_t zero[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) zero[k] = 0u;
+    for (int c = 0; c < ntask * (vssp::kTask / 16); ++c) tc::tmem_st16(tcol + 16 * c, zero);
+    tc::tmem_wait_st();
+}
+
+__device__ __noinline__ void vssp_flush(uint32_t tcol, int ntask, float4* to, bool add)
+{
+    using namespace vssp;
+    tc::tmem_wait_st();
+    for (int r = 0; r < ntask; ++r) {
+        for (int cc = 0; cc < N / 8; ++cc) {
+            float4* o = to + 8 * cc * NZ + r * NT;
+            float4 t[8];                                        // loads before the stores
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] = add ? __ldcg(o + k * NZ) : make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t u[16], q[16];
+            tc::tmem_ld16_issue(tcol + r * kTask + 16 * cc, u);
+            tc::tmem_ld16_issue(tcol + r * kTask + 2 * N + 16 * cc, q);
+            tc::tmem_wait();
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                __stcg(o + k * NZ, make_float4(__fadd_rn(t[k].x, __uint_as_float(u[2 * k])), __fadd_rn(t[k].y, __uint_as_float(u[2 * k + 1])),
+                                               __fadd_rn(t[k].z, __uint_as_float(q[2 * k])), __fadd_rn(t[k].w, __uint_as_float(q[2 * k + 1]))));
+        }
+    }
+}
 
 __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs a)
 {
@@ -118,15 +154,16 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
     };
 
     float4* F = reinterpret_cast<float4*>(a.F + size_t(blockIdx.x) * kF);      // [kx][ky*24 + kz]: (F0.re, F1.re, F0.im, F1.im)
-    const int Nrho = g.Nrho, M = g.M, ns = a.ns;
+    const int Nrho = g.Nrho, M = g.M;
     const float4* phase = static_cast<const float4*>(g.phase);
     const float* bself = static_cast<const float*>(g.bself);
     const float4* bcross = static_cast<const float4*>(g.bcross);
     const float2* c = static_cast<const float2*>(g.c);
-    const int64_t nitems = g.ndof * ns;
+    const int64_t nitems = split_items(g.ndof, a.plan);
     for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int64_t dof = item / ns;
-        const int part = int(item - dof * ns);
+        const SplitItem it = split_item(item, a.plan, Nrho);
+        const int64_t dof = it.li;
+        const int ns = it.ns;
         const float* f0 = static_cast<const float*>(g.f[0]) + dof * n;
         const float* f1 = static_cast<const float*>(g.f[1]) + dof * n;
 
@@ -165,18 +202,17 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
 #pragma unroll
             for (int k = 0; k < N; ++k)
                 F[k * NZ + t] = make_float4(vr[k].x * sc, vr[k].y * sc, vi[k].x * sc, vi[k].y * sc);
-            uint32_t zero[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) zero[k] = 0u;
-#pragma unroll
-            for (int k = 0; k < kTask / 16; ++k) tc::tmem_st16(tcol + r * kTask + 16 * k, zero);
         }
-        tc::tmem_wait_st();
 
         // ---- slices: radius rho, pair kind (0: species 0 with itself, 1: species 1
         // with itself, 2: unlike), direction s; phase tables kind by kind ----
-        const int rho1 = Nrho * (part + 1) / ns;
-        int rho = Nrho * part / ns, kind = 0, s = 0;
+        // G^ of a radius in tensor memory; at its end to the radius' slot (cut) or onto
+        // the sum of the radii
+        float4* Gs = ns > 1 ? reinterpret_cast<float4*>(a.slots + size_t(it.cut * Nrho) * kSlot)
+                            : reinterpret_cast<float4*>(a.sums + size_t(blockIdx.x) * kSlot);
+        const int rho1 = it.b1;
+        int rho = it.b0, kind = 0, s = 0;
+        vssp_clear(tcol, ntask);
         const int half = M / 2;
         auto table = [&](int q, int k, int d) { return (k < 2 ? (k * Nrho + q) * half : (Nrho + q) * M) + d; };
         if (tid < 3 * N) E[tid] = phase[size_t(table(rho, 0, 0)) * 3 * N + tid];
@@ -319,37 +355,22 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
                     }
                 }
             }
+            if (nrho != rho) {                                  // the radius' last slice
+                vssp_flush(tcol, ntask, (ns > 1 ? Gs + size_t(rho) * N * NZ : Gs) + tid, ns == 1 && rho > 0);
+                if (nrho < rho1) vssp_clear(tcol, ntask);
+            }
             rho = nrho;
             kind = nkind;
             s = ndir;
         }
-        tc::tmem_wait_st();
 
-        const float4* sum = nullptr;                            // parts' G^, when split
         if (ns > 1) {
-            float4* slot = reinterpret_cast<float4*>(a.slots + size_t(item) * kSlot);
-#pragma unroll 1
-            for (int r = 0; r < ntask; ++r) {
-#pragma unroll
-                for (int cc = 0; cc < N / 8; ++cc) {
-                    uint32_t u[16], q[16];
-                    tc::tmem_ld16_issue(tcol + r * kTask + 16 * cc, u);
-                    tc::tmem_ld16_issue(tcol + r * kTask + 2 * N + 16 * cc, q);
-                    tc::tmem_wait();
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        __stcg(slot + (8 * cc + k) * NZ + tid + r * NT,
-                               make_float4(__uint_as_float(u[2 * k]), __uint_as_float(u[2 * k + 1]),
-                                           __uint_as_float(q[2 * k]), __uint_as_float(q[2 * k + 1])));
-                }
-            }
             __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(a.tickets + dof, 1u) == uint32_t(ns - 1);
+            if (tid == 0) s_last = atomicAdd(a.tickets + it.cut, 1u) == uint32_t(ns - 1);
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
-            sum = reinterpret_cast<const float4*>(a.slots + size_t(dof) * ns * kSlot);
         }
 
         // ---- back to velocity space: lane A QG_p, lane B QL_p; Q_p = QG_p - f_p QL_p ----
@@ -359,30 +380,15 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
             for (int r = 0; r < ntask; ++r) {
                 const int t = tid + r * NT;
                 float2 vr[N], vi[N];
-                if (sum) {
-#pragma unroll
-                    for (int k = 0; k < N; ++k) vr[k].x = vi[k].x = 0.f;
+                // radii in order
 #pragma unroll 1
-                    for (int j = 0; j < ns; ++j) {
-                        const float2* sj = reinterpret_cast<const float2*>(sum + size_t(j) * N * NZ);
+                for (int j = 0; j < (ns > 1 ? Nrho : 1); ++j) {
+                    const float2* sj = reinterpret_cast<const float2*>(Gs + size_t(j) * N * NZ);
 #pragma unroll
-                        for (int k = 0; k < N; ++k) {
-                            const float2 v = __ldcg(sj + 2 * (k * NZ + t) + p);
-                            vr[k].x += v.x;
-                            vi[k].x += v.y;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int cc = 0; cc < N / 8; ++cc) {
-                        uint32_t u[16];
-                        tc::tmem_ld16_issue(tcol + r * kTask + p * 2 * N + 16 * cc, u);
-                        tc::tmem_wait();
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            vr[8 * cc + k].x = __uint_as_float(u[2 * k]);
-                            vi[8 * cc + k].x = __uint_as_float(u[2 * k + 1]);
-                        }
+                    for (int k = 0; k < N; ++k) {
+                        const float2 v = __ldcg(sj + 2 * (k * NZ + t) + p);
+                        vr[k].x = j ? __fadd_rn(vr[k].x, v.x) : v.x;
+                        vi[k].x = j ? __fadd_rn(vi[k].x, v.y) : v.y;
                     }
                 }
 #pragma unroll
@@ -433,8 +439,8 @@ static size_t vssp_head(int64_t nslots) { return (size_t(nslots + 1) * sizeof(ui
 extern "C" int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas)
 {
     if (nctas < 1) return 0;
-    // one F and two slots per CTA
-    return int64_t(vssp_head(2 * int64_t(nctas)) + size_t(nctas) * (vssp::kF + 2 * vssp::kSlot) + 256);
+    // F and the sum per CTA, and seven slots for the radii of cut distributions
+    return int64_t(vssp_head(7 * int64_t(nctas)) + size_t(nctas) * (vssp::kF + 8 * vssp::kSlot) + 256);
 }
 
 extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* scratch, int64_t bytes, void* stream)
@@ -451,24 +457,25 @@ extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* sc
     // CTAs and slots that fit
     const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
     const int64_t room = bytes - int64_t(base - reinterpret_cast<uintptr_t>(scratch));
-    int64_t nctas = std::min<int64_t>(nsm, (room - int64_t(vssp_head(0))) / int64_t(kF));
+    int64_t nctas = std::min<int64_t>(nsm, (room - int64_t(vssp_head(0))) / int64_t(kF + kSlot));
     if (nctas < 1) return BDGFS_ESCRATCH;
     int64_t nslots = 0;
-    while (int64_t(vssp_head(nslots + 1) + size_t(nctas) * kF + size_t(nslots + 1) * kSlot) <= room &&
-           nslots < 4 * int64_t(nsm))
+    while (int64_t(vssp_head(nslots + 1) + size_t(nctas) * (kF + kSlot) + size_t(nslots + 1) * kSlot) <= room &&
+           nslots < 7 * int64_t(nsm))
         ++nslots;
     VssPairArgs a{};
     a.g = *g;
-    a.ns = split_parts(g->ndof, nslots, g->Nrho, int(nctas), 0.3f, 0.4f);
+    a.plan = split_plan(g->ndof, nslots, g->Nrho, int(nctas), 0.3f, 0.4f);
     a.timeout = reinterpret_cast<uint32_t*>(base);
     a.tickets = a.timeout + 1;
     a.F = reinterpret_cast<unsigned char*>(base + vssp_head(nslots));
-    a.slots = a.F + size_t(nctas) * kF;
+    a.sums = a.F + size_t(nctas) * kF;
+    a.slots = a.sums + size_t(nctas) * kSlot;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(a.timeout, 0, sizeof(uint32_t) * (1 + (a.ns > 1 ? size_t(g->ndof) : 0)), st) != cudaSuccess)
+    if (cudaMemsetAsync(a.timeout, 0, sizeof(uint32_t) * (1 + size_t(g->ndof - a.plan.whole)), st) != cudaSuccess)
         return BDGFS_ECUDA;
     if (const int rc = smem_optin(reinterpret_cast<const void*>(vss_pair_kernel), kSmem)) return rc;
-    nctas = std::min(nctas, g->ndof * a.ns);
+    nctas = std::min(nctas, split_items(g->ndof, a.plan));
     vss_pair_kernel<<<unsigned(nctas), NT, kSmem, st>>>(a);
     return cuda_status(cudaGetLastError());
 }
