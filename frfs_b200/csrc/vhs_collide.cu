@@ -1285,6 +1285,7 @@ __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict_
 }
 
 }  // namespace bdgfs
+#include "vhs_exact.cuh"
 #include "vhs_tree.cuh"
 namespace bdgfs {
 
@@ -1448,6 +1449,19 @@ static size_t per_tree(int maxM, size_t* smem)
     return QLayoutTree::scratch_bytes();
 }
 
+template <typename T, int N>
+static int launch_exact(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                        int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                        uint64_t* counter, cudaStream_t st);
+
+template <typename T, int N>
+static size_t per_exact(int maxM, size_t* smem)
+{
+    *smem = Exact<T, N>::smem_bytes(maxM);
+    return Exact<T, N>::scratch_bytes();
+}
+
+#define ENTRYX(FP, T, N, MAXM) {FP, N, 0, Exact<T, N>::NT, &launch_exact<T, N>, &per_exact<T, N>, MAXM}
 #define VARIANT(T, N, NT, WG, SG) Variant<T, N, NT, WG, SG>
 #define VARIANTG(T, N, NT, GR) Variant<T, N, NT, false, false, GR>
 #define VARIANTS(T, NT) Variant<T, 32, NT, true, false, 0, true>
@@ -1507,6 +1521,13 @@ static const Entry kEntries[] = {
      &entry_per_cta<float, 320, VariantP2<true, true, true>, NoVariant>},
     // 24^3 by axis-wise shifts shared between directions (vhs_tree.cuh)
     {0, 24, 0, tree::NT, &launch_tree, &per_tree, tree::kMaxM},
+    // small grids, the Nyquist term from its planes (vhs_exact.cuh)
+    ENTRYX(0, float, 16, 0),
+    ENTRYX(0, float, 12, 0),
+    ENTRYX(0, float, 8, 0),
+    ENTRYX(1, double, 16, 48),                      // phases and planes in 227 KB
+    ENTRYX(1, double, 12, 0),
+    ENTRYX(1, double, 8, 0),
 };
 static constexpr int kNumEntries = int(sizeof(kEntries) / sizeof(kEntries[0]));
 
@@ -1648,6 +1669,28 @@ static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_
     const size_t smem = QLayoutTree::smem_bytes(a.g.M);
     if (const int rc = smem_optin(reinterpret_cast<const void*>(vhs_tree_kernel), smem)) return rc;
     vhs_tree_kernel<<<unsigned(nblk), tree::NT, smem, st>>>(a);
+    return cuda_status(cudaGetLastError());
+}
+
+template <typename T, int N>
+static int launch_exact(const bdgfs_vhs_grid* grids, int, const bdgfs_vhs_batch* batches, int nbatch, int flags,
+                        void* scratch, size_t scratch_bytes, uint64_t* counter, cudaStream_t st)
+{
+    using X = Exact<T, N>;
+    auto k = vhs_exact_kernel<T, N>;
+    const size_t smem = X::smem_bytes(grids[0].M);
+    if (const int rc = smem_optin(reinterpret_cast<const void*>(k), smem)) return rc;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, X::NT, smem) != cudaSuccess || occ < 1)
+        return BDGFS_ECUDA;
+    ExactArgs a{};
+    int64_t nblk = 0;
+    unsigned char* none = nullptr;
+    if (const int rc = split_launch(a, grids, batches, nbatch, flags, scratch, scratch_bytes, counter, 0,
+                                    X::slot_bytes(), std::min(occ, X::kCtas), 0.5f, 0.6f, st, &nblk, &none))
+        return rc;
+    if (nblk == 0) return BDGFS_OK;
+    k<<<unsigned(nblk), X::NT, smem, st>>>(a);
     return cuda_status(cudaGetLastError());
 }
 
