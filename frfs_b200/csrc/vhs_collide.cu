@@ -1287,6 +1287,7 @@ __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict_
 }  // namespace bdgfs
 #include "vhs_exact.cuh"
 #include "vhs_tree.cuh"
+#include "vhs_tree32.cuh"
 namespace bdgfs {
 
 struct KArgs {
@@ -1443,6 +1444,16 @@ static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_
                        int nbatch, int flags, void* scratch, size_t scratch_bytes,
                        uint64_t* counter, cudaStream_t st);
 
+static int launch_tree32(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                         int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                         uint64_t* counter, cudaStream_t st);
+
+static size_t per_tree32(int maxM, size_t* smem)
+{
+    *smem = QLayoutTree32::smem_bytes(maxM);
+    return QLayoutTree32::scratch_bytes();
+}
+
 static size_t per_tree(int maxM, size_t* smem)
 {
     *smem = QLayoutTree::smem_bytes(maxM);
@@ -1521,6 +1532,8 @@ static const Entry kEntries[] = {
      &entry_per_cta<float, 320, VariantP2<true, true, true>, NoVariant>},
     // 24^3 by axis-wise shifts shared between directions (vhs_tree.cuh)
     {0, 24, 0, tree::NT, &launch_tree, &per_tree, tree::kMaxM},
+    // the same at 32^3 (vhs_tree32.cuh)
+    {0, 32, 0, tree32::NT, &launch_tree32, &per_tree32, tree32::kMaxM},
     // small grids, the Nyquist term from its planes (vhs_exact.cuh)
     ENTRYX(0, float, 16, 0),
     ENTRYX(0, float, 12, 0),
@@ -1669,6 +1682,27 @@ static int launch_tree(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_
     const size_t smem = QLayoutTree::smem_bytes(a.g.M);
     if (const int rc = smem_optin(reinterpret_cast<const void*>(vhs_tree_kernel), smem)) return rc;
     vhs_tree_kernel<<<unsigned(nblk), tree::NT, smem, st>>>(a);
+    return cuda_status(cudaGetLastError());
+}
+
+// The same at 32^3; the exact-Nyquist mode runs on the warp-slab variant.
+static int launch_tree32(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch* batches,
+                         int nbatch, int flags, void* scratch, size_t scratch_bytes,
+                         uint64_t* counter, cudaStream_t st)
+{
+    if (flags & BDGFS_EXACT)
+        return launch<float, 256, VARIANTS(float, 256), NoVariant>(grids, ngrids, batches, nbatch, flags, scratch,
+                                                                   scratch_bytes, counter, st);
+    if (scratch_bytes < VARIANTS(float, 256)::L::scratch_bytes()) return BDGFS_ESCRATCH;
+    Tree32Args a{};
+    int64_t nblk = 0;
+    if (const int rc = split_launch(a, grids, batches, nbatch, flags, scratch, scratch_bytes, counter, tree32::kPriv,
+                                    QLayoutTree32::slot_bytes(), 1, 1.5f, 1.7f, st, &nblk, &a.priv))
+        return rc;
+    if (nblk == 0) return BDGFS_OK;
+    const size_t smem = QLayoutTree32::smem_bytes(a.g.M);
+    if (const int rc = smem_optin(reinterpret_cast<const void*>(vhs_tree32_kernel), smem)) return rc;
+    vhs_tree32_kernel<<<unsigned(nblk), tree32::NT, smem, st>>>(a);
     return cuda_status(cudaGetLastError());
 }
 
