@@ -30,22 +30,62 @@ __device__ __forceinline__ uint32_t mix32(uint64_t x)
     return uint32_t(x >> 32);
 }
 
-// NVC > 0: the grid size at compile time (h.Nv == NVC)
-template <typename T, int VEC, int NVC = 0>
-__global__ void __launch_bounds__(256, NVC > 0 ? 5 : 0) indicator_kernel(const bdgfs_hybrid_args h,
-                                                                         const T* __restrict__ f)
+// Lists and per-row scalars of row dof (one thread): density, drift u, temperature
+// Tt, e0 = |f - M|^2, e1 = |f|^2.  Returns the compact surrogate row or -1.
+__device__ inline int64_t indicate(const bdgfs_hybrid_args& h, int64_t dof, bool ok, double rho, double ux,
+                                   double uy, double uz, double Tt, double e0, double e1)
+{
+    int64_t pos = -1;
+    const double eps = (ok && e1 > 0.0) ? sqrt(e0 / e1) : 1e30;
+    if (h.eps) h.eps[dof] = float(eps);
+    const bool sur = eps < double(h.threshold);
+    const uint64_t seed = h.seed_dev ? *h.seed_dev : h.seed;
+    const bool re = sur && (double(mix32(seed * 0x100000001B3ull + uint64_t(dof))) <
+                            double(h.recheck) * 4294967296.0);
+    if (h.flag) h.flag[dof] = uint8_t(sur ? (re ? 2 : 1) : 0);
+    if (sur) {
+        const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts), 1ull));
+        h.sur_idx[p] = int32_t(dof);
+        h.sur_inv_rho[p] = float(1.0 / rho);
+        h.sur_rho2[p] = float(rho * rho);
+        pos = p;
+        if (h.sur_s) h.sur_s[p] = float(sqrt(e0) / rho);
+        if (h.sur_uT) {
+            h.sur_uT[4 * p + 0] = float(ux);
+            h.sur_uT[4 * p + 1] = float(uy);
+            h.sur_uT[4 * p + 2] = float(uz);
+            h.sur_uT[4 * p + 3] = float(Tt);
+        }
+        if (h.feat) {
+            __nv_bfloat16* fr = static_cast<__nv_bfloat16*>(h.feat) + p * h.feat_ld;
+            fr[0] = __float2bfloat16_rn(h.center ? 0.f : float(ux));
+            fr[1] = __float2bfloat16_rn(h.center ? 0.f : float(uy));
+            fr[2] = __float2bfloat16_rn(h.center ? 0.f : float(uz));
+            fr[3] = __float2bfloat16_rn(float(Tt - 1.0));
+        }
+    }
+    if (!sur || re) {
+        const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 1), 1ull));
+        h.spec_idx[p] = int32_t(dof);
+    }
+    if (re) atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 2), 1ull);
+    return pos;
+}
+
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256) indicator_kernel(const bdgfs_hybrid_args h, const T* __restrict__ f)
 {
     __shared__ double red[8 * 8];
     __shared__ double cs[kMaxNv], ex[3][kMaxNv];
     __shared__ int64_t s_pos;
     const int64_t dof = blockIdx.x;
-    const int Nv = NVC > 0 ? NVC : h.Nv;
+    const int Nv = h.Nv;
     const int n = Nv * Nv * Nv;
     const T* fd = f + dof * int64_t(n);
     for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = h.c0[i];
     __syncthreads();
     double m[5] = {0, 0, 0, 0, 0};
-    row_moments<T, VEC, NVC>(fd, n, Nv, cs, m);
+    row_moments<T, VEC>(fd, n, Nv, cs, m);
     block_sum<5>(m, red);
     const double rho = m[0] * h.cw;
     const double ux = m[1] / m[0], uy = m[2] / m[0], uz = m[3] / m[0];
@@ -69,7 +109,7 @@ __global__ void __launch_bounds__(256, NVC > 0 ? 5 : 0) indicator_kernel(const b
             Chunk<T, VEC> c;
             c.load(fd + v);
             uint32_t ix, iy, iz;
-            vsplit<NVC>(uint32_t(v), uint32_t(Nv), ix, iy, iz);
+            vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
             const double axy = a * ex[0][ix] * ex[1][iy];
 #pragma unroll
             for (int j = 0; j < VEC; ++j) {
@@ -81,42 +121,7 @@ __global__ void __launch_bounds__(256, NVC > 0 ? 5 : 0) indicator_kernel(const b
         }
     }
     block_sum<2>(e, red);
-    if (threadIdx.x == 0) {
-        const double eps = (ok && e[1] > 0.0) ? sqrt(e[0] / e[1]) : 1e30;
-        s_pos = -1;
-        if (h.eps) h.eps[dof] = float(eps);
-        const bool sur = eps < double(h.threshold);
-        const uint64_t seed = h.seed_dev ? *h.seed_dev : h.seed;
-        const bool re = sur && (double(mix32(seed * 0x100000001B3ull + uint64_t(dof))) <
-                                double(h.recheck) * 4294967296.0);
-        if (h.flag) h.flag[dof] = uint8_t(sur ? (re ? 2 : 1) : 0);
-        if (sur) {
-            const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts), 1ull));
-            h.sur_idx[p] = int32_t(dof);
-            h.sur_inv_rho[p] = float(1.0 / rho);
-            h.sur_rho2[p] = float(rho * rho);
-            s_pos = p;
-            if (h.sur_s) h.sur_s[p] = float(sqrt(e[0]) / rho);
-            if (h.sur_uT) {
-                h.sur_uT[4 * p + 0] = float(ux);
-                h.sur_uT[4 * p + 1] = float(uy);
-                h.sur_uT[4 * p + 2] = float(uz);
-                h.sur_uT[4 * p + 3] = float(Tt);
-            }
-            if (h.feat) {
-                __nv_bfloat16* fr = static_cast<__nv_bfloat16*>(h.feat) + p * h.feat_ld;
-                fr[0] = __float2bfloat16_rn(h.center ? 0.f : float(ux));
-                fr[1] = __float2bfloat16_rn(h.center ? 0.f : float(uy));
-                fr[2] = __float2bfloat16_rn(h.center ? 0.f : float(uz));
-                fr[3] = __float2bfloat16_rn(float(Tt - 1.0));
-            }
-        }
-        if (!sur || re) {
-            const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 1), 1ull));
-            h.spec_idx[p] = int32_t(dof);
-        }
-        if (re) atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 2), 1ull);
-    }
+    if (threadIdx.x == 0) s_pos = indicate(h, dof, ok, rho, ux, uy, uz, Tt, e[0], e[1]);
     __syncthreads();
     const int64_t p = s_pos;
     if (p >= 0 && h.dev_rows) {
@@ -129,7 +134,7 @@ __global__ void __launch_bounds__(256, NVC > 0 ? 5 : 0) indicator_kernel(const b
             Chunk<T, VEC> c;
             c.load(fd + v);
             uint32_t ix, iy, iz;
-            vsplit<NVC>(uint32_t(v), uint32_t(Nv), ix, iy, iz);
+            vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
             const double axy = a * ex[0][ix] * ex[1][iy];
             float d[VEC];
 #pragma unroll
@@ -143,6 +148,144 @@ __global__ void __launch_bounds__(256, NVC > 0 ? 5 : 0) indicator_kernel(const b
                 out[v] = __float2bfloat16_rn(d[0]);
             }
         }
+    }
+}
+
+// A row of N^3 FP32 values staged in shared memory, where every thread reads only
+// what it copied itself (no barrier): PL x-planes at a time, so a thread keeps
+// its y and its four z and only x moves (x = x0 + PL j).
+template <int N>
+struct OwnRow {
+    static constexpr int CP = N * N / 4;                       // chunks of four z per plane
+    static constexpr int PL = N == 16 ? 4 : 2, NT = PL * CP, NJ = N / PL;
+    static constexpr int CTAS = N == 24 ? 4 : 5;               // per SM
+    static constexpr size_t kSmem = size_t(N) * N * N * sizeof(float);
+    static_assert(NT % 32 == 0 && N % PL == 0, "whole warps and rounds");
+    int x0, y, z0;
+    const float* own;                                          // + 4 j NT: chunk j
+
+    __device__ __forceinline__ OwnRow(float* sh, const float* row)
+    {
+        const int t = threadIdx.x, r = t % CP;
+        x0 = t / CP;
+        y = r / (N / 4);
+        z0 = 4 * (r - y * (N / 4));
+        own = sh + 4 * t;
+        const uint32_t s = uint32_t(__cvta_generic_to_shared(sh + 4 * t));
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s + 16 * j * NT), "l"(row + 4 * (j * NT + t))
+                         : "memory");
+    }
+    __device__ __forceinline__ void wait() const { asm volatile("cp.async.wait_all;" ::: "memory"); }
+    __device__ __forceinline__ float4 at(int j) const { return *reinterpret_cast<const float4*>(own + 4 * j * NT); }
+    // FP64 moments {1, c, |c|^2}: sums over x per z value and over z per x, so a
+    // value costs one conversion and two additions
+    __device__ __forceinline__ void moments(const double* cs, double (&m)[5]) const
+    {
+        double A[4] = {0, 0, 0, 0}, B = 0, C = 0;
+#pragma unroll 4
+        for (int j = 0; j < NJ; ++j) {
+            const double cx = cs[x0 + PL * j];
+            const float4 v = at(j);
+            const double x[4] = {double(v.x), double(v.y), double(v.z), double(v.w)};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) A[k] += x[k];
+            const double b = (x[0] + x[1]) + (x[2] + x[3]), cb = cx * b;
+            B += cb;
+            C += cx * cb;
+        }
+        const double cy = cs[y];
+        m[0] = (A[0] + A[1]) + (A[2] + A[3]);
+        m[1] = B;
+        m[2] = cy * m[0];
+        double s1 = 0, s2 = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double cz = cs[z0 + k], t = cz * A[k];
+            s1 += t;
+            s2 += cz * t;
+        }
+        m[3] = s1;
+        m[4] = C + cy * m[2] + s2;
+    }
+};
+
+// indicator_kernel with the row in shared memory: f is read once and the index and
+// coordinate work is per thread, not per chunk.  3001 rows of 24^3, one B200: 123 ->
+// 74 us (3.4 TB/s).  Four CTAs (36 warps) an SM; with the row in registers 96
+// registers leave two (121 us; 95 with the next row's copy in flight).  Bound: the
+// latency of the chain sums -> parameters -> deviation -> list entry at that occupancy,
+// and the FP32 -> FP64 conversions.  At 32^3 a row fills an SM's shared memory (one
+// CTA), so the streaming kernel stays.
+template <int N>
+__global__ void __launch_bounds__(OwnRow<N>::NT, OwnRow<N>::CTAS)
+    indicator_own_kernel(const bdgfs_hybrid_args h, const float* __restrict__ f)
+{
+    using R = OwnRow<N>;
+    constexpr int n = N * N * N;
+    extern __shared__ __align__(16) float sh[];
+    __shared__ double red[5 * (R::NT / 32)];
+    __shared__ double cs[N], ex[3][N];
+    __shared__ int64_t s_pos;
+    const int64_t dof = blockIdx.x;
+    const R r(sh, f + dof * int64_t(n));
+    if (threadIdx.x < N) cs[threadIdx.x] = h.c0[threadIdx.x];
+    __syncthreads();
+    r.wait();
+    double m[5];
+    r.moments(cs, m);
+    block_sum<5>(m, red);
+    const double rho = m[0] * h.cw;
+    const double ux = m[1] / m[0], uy = m[2] / m[0], uz = m[3] / m[0];
+    const double Tt = (m[4] / m[0] - (ux * ux + uy * uy + uz * uz)) * (2.0 / 3.0);
+    const bool ok = rho > 0.0 && Tt > 0.0;
+    // separable Maxwellian: M = ex[0][ix] * ex[1][iy] * ex[2][iz]
+    if (ok && threadIdx.x < 3 * N) {
+        const int d = threadIdx.x / N, j = threadIdx.x - d * N;
+        const double c = cs[j] - (d == 0 ? ux : d == 1 ? uy : uz);
+        const double b = 3.141592653589793 * Tt, a = d == 0 ? rho / (b * sqrt(b)) : 1.0;
+        ex[d][j] = a * exp(-c * c / Tt);
+    }
+    __syncthreads();
+    double e[2] = {0, 0};
+    double ey = 0.0, ez[4] = {0, 0, 0, 0};
+    if (ok) {
+        ey = ex[1][r.y];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ez[k] = ex[2][r.z0 + k];
+#pragma unroll 4
+        for (int j = 0; j < R::NJ; ++j) {
+            const double axy = ex[0][r.x0 + R::PL * j] * ey;
+            const float4 v = r.at(j);
+            const double x[4] = {double(v.x), double(v.y), double(v.z), double(v.w)};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double d = x[k] - axy * ez[k];
+                e[0] += d * d;
+                e[1] += x[k] * x[k];
+            }
+        }
+    }
+    block_sum<2>(e, red);
+    if (threadIdx.x == 0) s_pos = indicate(h, dof, ok, rho, ux, uy, uz, Tt, e[0], e[1]);
+    __syncthreads();
+    const int64_t p = s_pos;
+    if (p < 0 || !h.dev_rows) return;                  // uniform per block
+    // (f - M[f]) / |f - M[f]|_2: direction of the deviation from the local
+    // Maxwellian (its size, at unit density, is sur_s)
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(h.dev_rows) + p * int64_t(n);
+    const double inv = (ok && e[0] > 0.0) ? 1.0 / sqrt(e[0]) : 0.0;
+#pragma unroll 4
+    for (int j = 0; j < R::NJ; ++j) {
+        const double axy = ok ? ex[0][r.x0 + R::PL * j] * ey : 0.0;
+        const float4 v = r.at(j);
+        const double x[4] = {double(v.x), double(v.y), double(v.z), double(v.w)};
+        float d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) d[k] = ok ? float((x[k] - axy * ez[k]) * inv) : 0.f;
+        __align__(8) __nv_bfloat162 hv[2] = {__floats2bfloat162_rn(d[0], d[1]), __floats2bfloat162_rn(d[2], d[3])};
+        *reinterpret_cast<uint2*>(out + 4 * (j * R::NT + int(threadIdx.x))) = *reinterpret_cast<const uint2*>(hv);
     }
 }
 
@@ -295,6 +438,82 @@ __global__ void __launch_bounds__(256) project_scatter_kernel(const bdgfs_hybrid
         }
     }
     if (!re) return;                                   // uniform per block
+    block_sum<2>(e, red);
+    if (threadIdx.x == 0 && h.recheck_err) {
+        atomicAdd(h.recheck_err, e[0]);
+        atomicAdd(h.recheck_err + 1, e[1]);
+    }
+}
+
+// project_scatter_kernel with the row in shared memory: Qc is read once.  3001 rows
+// of 24^3, one B200: 98 -> 64 us (5.2 TB/s; 84 with the row in registers).  Bound: HBM.
+template <int N>
+__global__ void __launch_bounds__(OwnRow<N>::NT, OwnRow<N>::CTAS)
+    project_scatter_own_kernel(const bdgfs_hybrid_args h, const float* __restrict__ Qc, float* __restrict__ Q)
+{
+    using R = OwnRow<N>;
+    constexpr int n = N * N * N;
+    extern __shared__ __align__(16) float sh[];
+    __shared__ double red[5 * (R::NT / 32)];
+    __shared__ double cs[N], lam[5];
+    const int64_t row = blockIdx.x;
+    if (row == 0 && threadIdx.x == 0 && h.seed_dev) *h.seed_dev += 1;   // next step's sample
+    const int64_t cnt = *h.counts;
+    if (row >= cnt) return;
+    const R r(sh, Qc + row * int64_t(n));
+    const int64_t dof = h.sur_idx[row];
+    const bool re = h.flag[dof] == 2;
+    if (threadIdx.x < N) cs[threadIdx.x] = h.c0[threadIdx.x];
+    __syncthreads();
+    r.wait();
+    double m[5];
+    r.moments(cs, m);
+    block_sum<5>(m, red);
+    // a non-finite row: as project_scatter_kernel
+    if (!isfinite(m[0] + m[1] + m[2] + m[3] + m[4])) {
+        if (!re && h.fb_idx && threadIdx.x == 0)
+            h.fb_idx[atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 3), 1ull)] = int32_t(dof);
+        return;
+    }
+    if (threadIdx.x < 5) {
+        double t = 0.0;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) t += h.ginv[threadIdx.x * 5 + j] * m[j];
+        lam[threadIdx.x] = t;
+    }
+    __syncthreads();
+    const double cy = cs[r.y], ly = lam[0] + lam[2] * cy + lam[4] * cy * cy;
+    double lz[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double cz = cs[r.z0 + k];
+        lz[k] = lam[3] * cz + lam[4] * cz * cz;
+    }
+    auto corrected = [&](int j) {
+        const double cx = cs[r.x0 + R::PL * j], l = ly + lam[1] * cx + lam[4] * cx * cx;
+        const float4 v = r.at(j);
+        return make_float4(float(double(v.x) - (l + lz[0])), float(double(v.y) - (l + lz[1])),
+                           float(double(v.z) - (l + lz[2])), float(double(v.w) - (l + lz[3])));
+    };
+    float4* dst = reinterpret_cast<float4*>(Q + dof * int64_t(n)) + threadIdx.x;
+    if (!re) {                                         // uniform per block
+#pragma unroll 4
+        for (int j = 0; j < R::NJ; ++j) dst[j * R::NT] = corrected(j);
+        return;
+    }
+    double e[2] = {0, 0};
+#pragma unroll 2
+    for (int j = 0; j < R::NJ; ++j) {
+        const float4 v = corrected(j), sp = dst[j * R::NT];
+        const double d[4] = {double(v.x) - double(sp.x), double(v.y) - double(sp.y),
+                             double(v.z) - double(sp.z), double(v.w) - double(sp.w)};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[0] += d[k] * d[k];
+        e[1] += double(sp.x) * double(sp.x);
+        e[1] += double(sp.y) * double(sp.y);
+        e[1] += double(sp.z) * double(sp.z);
+        e[1] += double(sp.w) * double(sp.w);
+    }
     block_sum<2>(e, red);
     if (threadIdx.x == 0 && h.recheck_err) {
         atomicAdd(h.recheck_err, e[0]);
@@ -467,43 +686,10 @@ __global__ void __launch_bounds__(256) indicator_smem_kernel(const bdgfs_hybrid_
     }
     block_sum<2>(e, red);
     if (threadIdx.x == 0) {
-        const double eps = (ok && e[1] > 0.0) ? sqrt(e[0] / e[1]) : 1e30;
-        s_pos = -1;
-        if (h.eps) h.eps[dof] = float(eps);
-        const bool sur = eps < double(h.threshold);
-        const uint64_t seed = h.seed_dev ? *h.seed_dev : h.seed;
-        const bool re = sur && (double(mix32(seed * 0x100000001B3ull + uint64_t(dof))) <
-                                double(h.recheck) * 4294967296.0);
-        if (h.flag) h.flag[dof] = uint8_t(sur ? (re ? 2 : 1) : 0);
-        if (sur) {
-            const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts), 1ull));
-            h.sur_idx[p] = int32_t(dof);
-            h.sur_inv_rho[p] = float(1.0 / rho);
-            h.sur_rho2[p] = float(rho * rho);
-            s_pos = p;
-            if (h.sur_s) h.sur_s[p] = float(sqrt(e[0]) / rho);
-            if (h.sur_uT) {
-                h.sur_uT[4 * p + 0] = float(ux);
-                h.sur_uT[4 * p + 1] = float(uy);
-                h.sur_uT[4 * p + 2] = float(uz);
-                h.sur_uT[4 * p + 3] = float(Tt);
-            }
-            if (h.feat) {
-                __nv_bfloat16* fr = static_cast<__nv_bfloat16*>(h.feat) + p * h.feat_ld;
-                fr[0] = __float2bfloat16_rn(h.center ? 0.f : float(ux));
-                fr[1] = __float2bfloat16_rn(h.center ? 0.f : float(uy));
-                fr[2] = __float2bfloat16_rn(h.center ? 0.f : float(uz));
-                fr[3] = __float2bfloat16_rn(float(Tt - 1.0));
-            }
-            s_u[0] = float(ux);
-            s_u[1] = float(uy);
-            s_u[2] = float(uz);
-        }
-        if (!sur || re) {
-            const int64_t p = int64_t(atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 1), 1ull));
-            h.spec_idx[p] = int32_t(dof);
-        }
-        if (re) atomicAdd(reinterpret_cast<unsigned long long*>(h.counts + 2), 1ull);
+        s_pos = indicate(h, dof, ok, rho, ux, uy, uz, Tt, e[0], e[1]);
+        s_u[0] = float(ux);
+        s_u[1] = float(uy);
+        s_u[2] = float(uz);
     }
     __syncthreads();
     const int64_t p = s_pos;
@@ -760,6 +946,14 @@ static int staged_project_scatter(const bdgfs_hybrid_args* h, const float* q, fl
     }
 }
 
+template <int N, typename K, typename... P>
+static int launch_own(K k, const bdgfs_hybrid_args* h, cudaStream_t st, P... p)
+{
+    if (const int rc = smem_optin(reinterpret_cast<const void*>(k), OwnRow<N>::kSmem)) return rc;
+    k<<<unsigned(h->ndof), OwnRow<N>::NT, OwnRow<N>::kSmem, st>>>(*h, p...);
+    return cuda_status(cudaGetLastError());
+}
+
 extern "C" int32_t bdgfs_hybrid_classify(const bdgfs_hybrid_args* h, const void* f, void* stream)
 {
     int rc = check_h(h);
@@ -788,8 +982,11 @@ extern "C" int32_t bdgfs_hybrid_classify(const bdgfs_hybrid_args* h, const void*
         else
             indicator_kernel<double, 1><<<unsigned(h->ndof), 256, 0, st>>>(*h, static_cast<const double*>(f));
     } else {
-        if (v4 && h->Nv == 24)
-            indicator_kernel<float, 4, 24><<<unsigned(h->ndof), 256, 0, st>>>(*h, static_cast<const float*>(f));
+        const float* fs = static_cast<const float*>(f);
+        if (v4 && h->Nv == 16)
+            return launch_own<16>(indicator_own_kernel<16>, h, st, fs);
+        else if (v4 && h->Nv == 24)
+            return launch_own<24>(indicator_own_kernel<24>, h, st, fs);
         else if (v4)
             indicator_kernel<float, 4><<<unsigned(h->ndof), 256, 0, st>>>(*h, static_cast<const float*>(f));
         else
@@ -859,7 +1056,13 @@ extern "C" int32_t bdgfs_hybrid_project_scatter(const bdgfs_hybrid_args* h, cons
             project_scatter_kernel<double, 1><<<unsigned(h->ndof), 256, 0, st>>>(
                 *h, static_cast<const double*>(Qc), static_cast<double*>(Q));
     } else {
-        if (v4)
+        const float* qs = static_cast<const float*>(Qc);
+        float* o = static_cast<float*>(Q);
+        if (v4 && h->Nv == 16)
+            return launch_own<16>(project_scatter_own_kernel<16>, h, st, qs, o);
+        else if (v4 && h->Nv == 24)
+            return launch_own<24>(project_scatter_own_kernel<24>, h, st, qs, o);
+        else if (v4)
             project_scatter_kernel<float, 4><<<unsigned(h->ndof), 256, 0, st>>>(
                 *h, static_cast<const float*>(Qc), static_cast<float*>(Q));
         else
