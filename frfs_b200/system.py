@@ -132,22 +132,19 @@ class DGFSElements:
         if ref == 0.0:
             return None
         kt = np.array([[m3[i * st[1], fid[0, j]] for j in range(p)] for i in range(p)])
-        kw = kt / kt[0, 0] if nd == 2 else None
-        if nd == 3:
-            kt = np.array([[m3[i * st[1], fid[0, j]] for j in range(p)] for i in range(p)])
-            kw = kt / kt[0, 0]
+        kw = kt / kt[0, 0]
         # scale so that kw is the factor itself (rows of K w sum like a quadrature
         # of the constant: sum_j kw[i][j] = 1)
         kw = kw / kw[0].sum()
         kn = np.array([[m3[i * st[0], f0[s]] for i in range(p)] for s in (0, 1)]) / kw[0, 0]**(nd - 1)
-        for f in range(nf):
-            d, side = int(np.argmax(np.abs(nref[f]))), int(nref[f].sum() > 0)
-            col = np.ones(nu)
-            for a in range(nd):
-                ua = (np.arange(nu) // st[a]) % p
-                col *= kn[side][ua] if a == d else kw[ua, (fsel[f] // st[a]) % p]
-            if not np.allclose(col, m3[:, f], rtol=0, atol=1e-12 * np.abs(m3).max()):
-                return None
+        fd = np.argmax(np.abs(nref), axis=1)                     # [nf] direction and side of a flux point
+        fs = (nref[np.arange(nf), fd] > 0).astype(int)
+        want = np.ones((nu, nf))
+        for a in range(nd):
+            ua = (np.arange(nu) // st[a]) % p
+            want *= np.where(fd == a, kn[fs][:, ua].T, kw[ua][:, (fsel // st[a]) % p])
+        if not np.allclose(want, m3, rtol=0, atol=1e-12 * np.abs(m3).max()):
+            return None
         self.af_fid = self.be.const(fid, dtype=torch.int32)
         self.af_smat = self.be.const(np.ascontiguousarray(S), dtype=self.be.fpdtype)
         a = _lib.FrAffine(fsel=self.fsel.data_ptr(), fid=self.af_fid.data_ptr(),
