@@ -19,7 +19,7 @@
 // group of eight rows.  G^ of both species stays in tensor memory.  F comes from
 // the CTA's scratch and the weights from their tables, through L2: 165 KB (like
 // pair) or 442 KB a slice.  Measured on one B200, Nrho = M = 12, 370 argon-krypton
-// pairs: 25.6 -> 10.9 ms (the general kernel of vss.cu -> this one; 12.3 ms before
+// pairs: 25.6 -> 10.5 ms (the general kernel of vss.cu -> this one; 12.3 ms before
 // the last round's distributions were cut over radii); error against 64-bit
 // arithmetic 4.0e-6 -> 3.5e-6 of Q.  Bound: the FP32 pipe and the barriers
 // between passes.  (The factors are real but for Nyquist terms; packing them as
@@ -87,6 +87,29 @@ __device__ __noinline__ void vssp_flush(uint32_t tcol, int ntask, float4* to, bo
                 __stcg(o + k * NZ, make_float4(__fadd_rn(t[k].x, __uint_as_float(u[2 * k])), __fadd_rn(t[k].y, __uint_as_float(u[2 * k + 1])),
                                                __fadd_rn(t[k].z, __uint_as_float(q[2 * k])), __fadd_rn(t[k].w, __uint_as_float(q[2 * k + 1]))));
         }
+    }
+}
+
+// The thread's pencils of the Nrho slots at ``from``, added in order into ``to``.  A
+// call of its own: inside the last stage its loop cost the slices 110 bytes of
+// spills (370 pairs: 10.9 -> 10.5 ms).
+__device__ __noinline__ void vssp_merge(const float4* from, float4* to, int Nrho, int ntask)
+{
+    using namespace vssp;
+    for (int r = 0; r < ntask; ++r, from += NT, to += NT) {
+        float4 s[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) s[k] = __ldcg(from + k * NZ);
+#pragma unroll 1
+        for (int j = 1; j < Nrho; ++j) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const float4 v = __ldcg(from + size_t(j) * N * NZ + k * NZ);
+                s[k] = make_float4(__fadd_rn(s[k].x, v.x), __fadd_rn(s[k].y, v.y), __fadd_rn(s[k].z, v.z), __fadd_rn(s[k].w, v.w));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k) __stcg(to + k * NZ, s[k]);
     }
 }
 
@@ -371,6 +394,9 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
+            float4* sum = reinterpret_cast<float4*>(a.sums + size_t(blockIdx.x) * kSlot);
+            vssp_merge(Gs + tid, sum + tid, Nrho, ntask);
+            Gs = sum;
         }
 
         // ---- back to velocity space: lane A QG_p, lane B QL_p; Q_p = QG_p - f_p QL_p ----
@@ -380,16 +406,12 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
             for (int r = 0; r < ntask; ++r) {
                 const int t = tid + r * NT;
                 float2 vr[N], vi[N];
-                // radii in order
-#pragma unroll 1
-                for (int j = 0; j < (ns > 1 ? Nrho : 1); ++j) {
-                    const float2* sj = reinterpret_cast<const float2*>(Gs + size_t(j) * N * NZ);
+                const float2* sp = reinterpret_cast<const float2*>(Gs) + 2 * t + p;
 #pragma unroll
-                    for (int k = 0; k < N; ++k) {
-                        const float2 v = __ldcg(sj + 2 * (k * NZ + t) + p);
-                        vr[k].x = j ? __fadd_rn(vr[k].x, v.x) : v.x;
-                        vi[k].x = j ? __fadd_rn(vi[k].x, v.y) : v.y;
-                    }
+                for (int k = 0; k < N; ++k) {
+                    const float2 v = __ldcg(sp + 2 * k * NZ);
+                    vr[k].x = v.x;
+                    vi[k].x = v.y;
                 }
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
