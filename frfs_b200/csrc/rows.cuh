@@ -119,7 +119,7 @@ __device__ __forceinline__ void chunk_moments(const Chunk<T, VEC>& c, double cx,
 }
 
 // FP64 raw moments {sum x, sum c x, sum |c|^2 x} of one row (block-wide)
-template <typename T, int VEC, int NVC = 0>
+template <typename T, int VEC>
 __device__ __forceinline__ void row_moments(const T* __restrict__ row, int n, int Nv, const double* cs,
                                             double (&m)[5])
 {
@@ -128,7 +128,7 @@ __device__ __forceinline__ void row_moments(const T* __restrict__ row, int n, in
         Chunk<T, VEC> c;
         c.load(row + v);
         uint32_t ix, iy, iz;
-        vsplit<NVC>(uint32_t(v), uint32_t(Nv), ix, iy, iz);
+        vsplit(uint32_t(v), uint32_t(Nv), ix, iy, iz);
         chunk_moments<T, VEC, 5>(c, cs[ix], cs[iy], cs + iz, m);
     }
 }
