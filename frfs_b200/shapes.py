@@ -103,6 +103,7 @@ class TensorShape:
         self.nfacefpts = nff
         self.nfpts = len(fp)
         self.facefpts = np.split(np.arange(self.nfpts), np.cumsum(nff)[:-1])
+        self._opmats = {}
 
     def nodal_at(self, pts):
         """Tensor Lagrange basis at pts: (npts, nupts) and its gradient
@@ -132,7 +133,7 @@ class TensorShape:
 
     @property
     def m2(self):
-        m0 = self.m0
+        m0 = self.opmat('M0')
         return np.concatenate([self.norm_fpts[:, a:a + 1] * m0
                                for a in range(self.ndims)], axis=1)
 
@@ -166,8 +167,10 @@ class TensorShape:
         return TensorShape(self.name, order).nodal_at(self.upts)[0]
 
     def opmat(self, expr):
-        mats = {'M0': self.m0, 'M1': self.m1, 'M2': self.m2, 'M3': self.m3,
-                'M12': self.m12}
-        if expr == 'M1 - M3*M2':
-            return mats['M1'] - mats['M3'] @ mats['M2']
-        return mats[expr]
+        """A copy of the operator, each built once per shape."""
+        if expr not in self._opmats:
+            if expr == 'M1 - M3*M2':
+                self._opmats[expr] = self.opmat('M1') - self.opmat('M3') @ self.opmat('M2')
+            else:
+                self._opmats[expr] = getattr(self, {'M0': 'm0', 'M1': 'm1', 'M2': 'm2', 'M3': 'm3', 'M12': 'm12'}[expr])
+        return self._opmats[expr].copy()

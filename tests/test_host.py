@@ -33,6 +33,22 @@ def test_operator_matrices_match_reference(kind, order):
     assert np.array_equal(s.norm_fpts, g['norm_fpts'])
 
 
+def test_operator_matrices_are_built_once(monkeypatch):
+    """Building a system's operators evaluates the nodal basis twice (at the
+    flux points and at the solution points), however many are asked for; what
+    a caller does to its copy stays its own."""
+    calls = []
+    real = TensorShape.nodal_at
+    monkeypatch.setattr(TensorShape, 'nodal_at', lambda self, pts: (calls.append(1), real(self, pts))[1])
+    s = TensorShape('hex', 2)
+    for m in ('M0', 'M1', 'M2', 'M1', 'M3', 'M1 - M3*M2', 'M3', 'M12'):
+        s.opmat(m)[...] = 7.0
+    assert len(calls) <= 2
+    assert np.array_equal(s.opmat('M0'), real(s, s.fpts)[0])
+    with pytest.raises(KeyError):
+        s.opmat('M9')
+
+
 class _Mesh:
     """An arbitrary affine element set (the golden metrics mesh)."""
 
