@@ -10,7 +10,7 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIBPATH = os.path.join(_HERE, '_lib', 'libbdgfs.so')
 
-BDGFS_OK = 0
+BDGFS_OK, BDGFS_EINVAL = 0, -1
 _ERRORS = {-1: 'invalid argument', -2: 'CUDA error', -3: 'unsupported grid/precision',
            -4: 'bounded device wait timed out', -5: 'scratch buffer too small'}
 

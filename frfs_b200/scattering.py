@@ -148,15 +148,24 @@ class VHSCollider:
         """batches: list of (grid_index, f[ndof, n], Q[ndof, n], moments|None).
         index (int32, device) / count (int64 device scalar) restrict the first
         batch to f[index[i]], i < count (read by the kernel)."""
-        if self._each is not None:
-            for gi, col in enumerate(self._each):
-                own = [(0,) + tuple(b[1:]) for b in batches if b[0] == gi]
-                if own:
-                    first = batches[0][0] == gi
-                    col(own, project, exact, stream, index if first else None, count if first else None)
+        bs = self._structs(batches, index, count)
+        flags = (1 if project else 0) | (2 if exact else 0)
+        if self._each is None:
+            self._launch(bs, flags, stream)
             return
-        L = _lib.lib()
-        bs = (_lib.VhsBatch * len(batches))()
+        # the checks of bdgfs_vhs_collide over the whole list, before any launch
+        if not 1 <= len(bs) <= 4 or any(not 0 <= b.grid < len(self.grids) for b in bs):
+            _lib.check(_lib.BDGFS_EINVAL, 'bdgfs_vhs_collide')
+        for gi, col in enumerate(self._each):
+            own = [b for b in bs if b.grid == gi]
+            for b in own:
+                b.grid = 0
+            if own:
+                col._launch(own, flags, stream)
+
+    def _structs(self, batches, index, count):
+        """The checked batches as C structures."""
+        bs = []
         for i, (gi, f, Q, mom) in enumerate(batches):
             g = self.grids[gi]
             n3 = g.Nv**3
@@ -171,22 +180,23 @@ class VHSCollider:
                 raise ValueError('moments must be float64 [ndof][10]')
             if f.device.type != 'cuda' or Q.device.type != 'cuda':
                 raise _lib.BdgfsError('f and Q must be CUDA tensors')
-            bs[i] = _lib.VhsBatch(grid=gi, ndof=f.numel() // n3, f=f.data_ptr(),
-                                  Q=Q.data_ptr(),
-                                  moments=mom.data_ptr() if mom is not None else 0)
+            b = _lib.VhsBatch(grid=gi, ndof=f.numel() // n3, f=f.data_ptr(), Q=Q.data_ptr(),
+                              moments=mom.data_ptr() if mom is not None else 0)
             if i == 0 and index is not None:
                 if index.dtype != torch.int32 or not index.is_cuda:
                     raise TypeError('index must be an int32 CUDA tensor')
-                bs[i].index = index.data_ptr()
+                b.index = index.data_ptr()
             if i == 0 and count is not None:
                 if count.dtype != torch.int64 or not count.is_cuda:
                     raise TypeError('count must be an int64 CUDA tensor')
-                bs[i].count = count.data_ptr()
-        rc = L.bdgfs_vhs_collide(self._garr, len(self.grids), bs, len(batches),
-                                 (1 if project else 0) | (2 if exact else 0),
-                                 _lib.ptr(self.scratch),
-                                 self.scratch.numel(), _lib.ptr(self.counter),
-                                 _lib.stream_ptr(stream))
+                b.count = count.data_ptr()
+            bs.append(b)
+        return bs
+
+    def _launch(self, bs, flags, stream):
+        rc = _lib.lib().bdgfs_vhs_collide(self._garr, len(self.grids), (_lib.VhsBatch * len(bs))(*bs), len(bs),
+                                          flags, _lib.ptr(self.scratch), self.scratch.numel(),
+                                          _lib.ptr(self.counter), _lib.stream_ptr(stream))
         _lib.check(rc, 'bdgfs_vhs_collide')
 
 

@@ -74,3 +74,28 @@ def test_tuner_tries_one_launch_per_grid(cuda, monkeypatch, tmp_path):
     q = [torch.empty_like(f) for f in fs]
     VHSCollider(again, cuda)([(0, fs[0], q[0], None), (1, fs[1], q[1], None)])
     assert all(bool(torch.isfinite(x).all()) for x in q)
+
+
+@pytest.mark.parametrize('by_grid', [False, True])
+def test_bad_lists_are_refused_before_any_launch(cuda, by_grid):
+    """A grid index outside the set, an empty list, too many batches, and a bad
+    second batch: the same errors in one launch and in one per grid, and nothing
+    written."""
+    from frfs_b200 import _lib
+    from frfs_b200.scattering import BY_GRID, VHSCollider
+    grids, fs = _grids()
+    for g in grids:
+        g.struct.tile = BY_GRID if by_grid else 0
+    col = VHSCollider(grids, cuda)
+    q = [torch.full_like(f, 7.0) for f in fs]
+    good = (0, fs[0], q[0], None)
+    bad = [([good, (2, fs[1], q[1], None)], IndexError), ([good, (-1, fs[1], q[1], None)], _lib.BdgfsError),
+           ([], _lib.BdgfsError), ([good] * 5, _lib.BdgfsError),
+           ([good, (1, fs[1], q[1].double(), None)], TypeError),
+           ([good, (1, fs[1][:, ::2], q[1], None)], ValueError),
+           ([good, (1, fs[1], q[1][:3], None)], ValueError)]
+    for batches, err in bad:
+        with pytest.raises(err):
+            col(batches)
+    torch.cuda.synchronize()
+    assert all(bool((x == 7.0).all()) for x in q)
