@@ -45,7 +45,7 @@ template <typename T>
 __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
 
 // Block-wide sum of NV doubles; every thread gets the result.
-// red must hold NV * (blockDim.x / 32) doubles.
+// red must hold NV * (blockDim.x / 32) doubles; blockDim.x is a multiple of 32.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* red)
 {

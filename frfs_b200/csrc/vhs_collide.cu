@@ -1324,6 +1324,7 @@ struct VariantP2 {
 template <typename T, int NT, typename V0, typename V1>
 __global__ void __launch_bounds__(NT, 1) __maxnreg__(65536 / NT / 8 * 8 > 255 ? 255 : 65536 / NT / 8 * 8) vhs_collide_kernel(const KArgs a)
 {
+    static_assert(NT % 32 == 0, "block_sum counts whole warps");
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int64_t s_item;
     __shared__ int64_t s_start[5];
@@ -1499,7 +1500,7 @@ static const Entry kEntries[] = {
     ENTRY1(0, float, 256, 16, false, false),
     ENTRY1(0, float, 128, 16, false, false),
     ENTRYG(0, float, 256, 16, 2),
-    ENTRY1(0, float, 144, 12, false, false),
+    ENTRY1(0, float, 160, 12, false, false),         // whole warps: block sums need them
     ENTRY1(0, float, 64, 8, false, false),
     // fp32, two grids in one launch
     ENTRY(0, float, 288, 24, false, false, 32, true, true),
@@ -1508,7 +1509,7 @@ static const Entry kEntries[] = {
     ENTRY1(1, double, 256, 16, false, false),
     ENTRY1(1, double, 128, 16, false, false),
     ENTRYG(1, double, 256, 16, 2),
-    ENTRY1(1, double, 144, 12, false, false),
+    ENTRY1(1, double, 160, 12, false, false),
     ENTRY1(1, double, 64, 8, false, false),
     // appended variants (earlier tile indices stay valid)
     ENTRY1(0, float, 384, 24, false, false),

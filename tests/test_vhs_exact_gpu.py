@@ -96,3 +96,28 @@ def test_exact_kernel_split(cuda, Nv, prec, n):
         assert float((r[done] - want[done]).norm() / want[done].norm()) < (1e-12 if prec == 'double' else 2e-5)
         rest = [i for i in range(n) if i not in done]
         assert not bool(r[rest].any())
+
+
+@pytest.mark.parametrize('prec', ['single', 'double'])
+@pytest.mark.parametrize('Nv', [8, 12, 16])
+def test_projection_of_every_variant(cuda, prec, Nv):
+    """Every compiled variant conserves mass, momentum and energy, by sums taken
+    outside the kernel, and gives the projected Q of the others.  The sums of Q
+    over n values: FP64 n eps = 1e-12 of their sum of magnitudes; FP32 one
+    rounding of each value (6e-8) at most.  Between variants: as without
+    projection."""
+    from frfs_b200.autotune import variants
+    from frfs_b200.scattering import VHSCollider
+    be, vm, sm, _ = _setup(Nv, 4, 6, prec)
+    f = _rows(vm, 3, be)
+    cv = vm.cv()
+    phi = np.stack([np.ones(cv.shape[1]), *cv, np.sum(cv * cv, axis=0)])
+    qs = []
+    for t in range(len(variants([sm.grid]))):
+        sm.grid.struct.tile = t
+        q = torch.full_like(f, float('nan'))
+        VHSCollider([sm.grid], be.device)([(0, f, q, None)], project=True, exact=True)
+        Q = q.double().cpu().numpy()
+        assert (np.abs(Q @ phi.T) <= (1e-12 if prec == 'double' else 1e-7) * (np.abs(Q) @ np.abs(phi).T)).all(), t
+        qs.append(q.double())
+        assert float((qs[-1] - qs[0]).norm() / qs[0].norm()) < (1e-12 if prec == 'double' else 5e-5), t
