@@ -218,49 +218,70 @@ __device__ __forceinline__ void shakov_heat(const double* u, double Pr, double (
                + (1.0 - Pr) * (-2.0 * Pu[i] + rho * v[i] * u2 - 1.5 * rho * Tt * v[i]);
 }
 
-constexpr int kRelaxWarps = 16;                        // threads per CTA: 256 or 512
+// partial sums that a row's moments are made of, with 256 or 512 threads: a row gives
+// the same bits alone and among thousands (512 slots, walked twice by 256 threads:
+// ARS-222 step of 2048 rows of 24^3 418 us; 256 slots: 380 us)
+constexpr int kRowSlots = 256, kRowWarps = kRowSlots / 32;
 
-// Moments of up to two rows in one walk (so both rows' loads are in flight
-// together); sums of row r in ms[r] (warp 0 writes them: read after the barrier)
+// Moments of up to two rows; sums of row r in ms[r] (warp 0 writes them: read after
+// the barrier).  256 threads walk both rows at once (both rows' loads are in flight
+// together); of 512, each half walks one row: a BDF-2 Shakov step of 315 rows 82 -> 74
+// us against every thread on both rows.
 template <typename T, int VEC, int NA>
 __device__ __forceinline__ void two_row_moments(const T* __restrict__ r0, const T* __restrict__ r1, int n, int Nv,
                                                 const double* cs, double cw, double (*red)[2][NA], double (*ms)[NA])
 {
-    double m0[NA], m1[NA];
-#pragma unroll
-    for (int i = 0; i < NA; ++i) m0[i] = m1[i] = 0.0;
-    RowWalk w(threadIdx.x * VEC, blockDim.x * VEC, uint32_t(Nv));
-#pragma unroll 2
-    for (int v = threadIdx.x * VEC; v < n; v += blockDim.x * VEC) {
-        Chunk<T, VEC> a, b;
-        if (r0) a.load(r0 + v);
-        if (r1) b.load(r1 + v);
-        if (r0) chunk_moments<T, VEC, NA>(a, cs[w.ix], cs[w.iy], cs + w.iz, m0);
-        if (r1) chunk_moments<T, VEC, NA>(b, cs[w.ix], cs[w.iy], cs + w.iz, m1);
-        w.next();
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < NA; ++i) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            if (r0) m0[i] += __shfl_xor_sync(0xffffffffu, m0[i], o);
-            if (r1) m1[i] += __shfl_xor_sync(0xffffffffu, m1[i], o);
-        }
-    }
-    if (lane == 0) {
+    const int slot = threadIdx.x & (kRowSlots - 1), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    RowWalk w(slot * VEC, kRowSlots * VEC, uint32_t(Nv));
+    auto warp_sums = [&](double (&m)[NA], int r) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
-            red[warp][0][i] = m0[i];
-            red[warp][1][i] = m1[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m[i] += __shfl_xor_sync(0xffffffffu, m[i], o);
         }
+        if (lane == 0) {
+#pragma unroll
+            for (int i = 0; i < NA; ++i) red[slot >> 5][r][i] = m[i];
+        }
+    };
+    if (blockDim.x > kRowSlots) {
+        const int r = threadIdx.x >= kRowSlots;
+        const T* row = r ? r1 : r0;
+        if (row) {
+            double m[NA];
+#pragma unroll
+            for (int i = 0; i < NA; ++i) m[i] = 0.0;
+#pragma unroll 4
+            for (int v = slot * VEC; v < n; v += kRowSlots * VEC) {
+                Chunk<T, VEC> a;
+                a.load(row + v);
+                chunk_moments<T, VEC, NA>(a, cs[w.ix], cs[w.iy], cs + w.iz, m);
+                w.next();
+            }
+            warp_sums(m, r);
+        }
+    } else {
+        double m0[NA], m1[NA];
+#pragma unroll
+        for (int i = 0; i < NA; ++i) m0[i] = m1[i] = 0.0;
+#pragma unroll 2
+        for (int v = slot * VEC; v < n; v += kRowSlots * VEC) {
+            Chunk<T, VEC> a, b;
+            if (r0) a.load(r0 + v);
+            if (r1) b.load(r1 + v);
+            if (r0) chunk_moments<T, VEC, NA>(a, cs[w.ix], cs[w.iy], cs + w.iz, m0);
+            if (r1) chunk_moments<T, VEC, NA>(b, cs[w.ix], cs[w.iy], cs + w.iz, m1);
+            w.next();
+        }
+        if (r0) warp_sums(m0, 0);
+        if (r1) warp_sums(m1, 1);
     }
     __syncthreads();
     if (warp == 0 && lane < NA) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             double s = 0.0;
-            for (int k = 0; k < int(blockDim.x >> 5); ++k) s += red[k][r][lane];
+            for (int k = 0; k < kRowWarps; ++k) s += red[k][r][lane];
             ms[r][lane] = s * cw;
         }
     }
@@ -269,10 +290,10 @@ __device__ __forceinline__ void two_row_moments(const T* __restrict__ r0, const 
 
 // moment rows alone (the same sums, in the same order, as inside the stage kernels)
 template <typename T, int VEC, int NA>
-__global__ void __launch_bounds__(512) row_moments_kernel(const T* __restrict__ f, int Nv, const double* c0, double cw,
+__global__ void __launch_bounds__(kRowSlots) row_moments_kernel(const T* __restrict__ f, int Nv, const double* c0, double cw,
                                                           double* __restrict__ U)
 {
-    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double red[kRowWarps][2][NA];
     __shared__ double ms[2][NA];
     __shared__ double cs[kMaxNv];
     const int64_t dof = blockIdx.x;
@@ -358,7 +379,7 @@ __device__ __forceinline__ double target_at(const Target& t, const double (*ex)[
 template <typename T, int VEC, int NA, int AR>
 __global__ void __launch_bounds__(512, NA == 5 && AR <= 2 ? 2 : 1) ars_kernel(const bdgfs_ars_args g)
 {
-    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double red[kRowWarps][2][NA];
     __shared__ double ms[2][NA];                       // moments of f_0 and of L_{ar-1}
     __shared__ double cs[kMaxNv];
     __shared__ double ex[NA == 11 ? 1 : 4][3][kMaxNv];
@@ -542,7 +563,7 @@ __global__ void __launch_bounds__(512, NA == 5 && AR <= 2 ? 2 : 1) ars_kernel(co
 template <typename T, int VEC, int NA, int BQ>
 __global__ void __launch_bounds__(512, NA == 5 ? 2 : 1) bdf_kernel(const bdgfs_bdf_args g)
 {
-    __shared__ double red[kRelaxWarps][2][NA];
+    __shared__ double red[kRowWarps][2][NA];
     __shared__ double ms[2][NA];                       // moments of f_{q-1} and of L_{q-1}
     __shared__ double cs[kMaxNv];
     __shared__ double ex[1][3][kMaxNv];
@@ -695,8 +716,7 @@ int32_t launch_moments(const void* f, int64_t ndof, int Nv, int fp64, const doub
                        cudaStream_t st)
 {
     const bool v4 = Nv % 4 == 0 && a16(f);
-    const unsigned nt = relax_threads(ndof);
-#define GO(T, V) row_moments_kernel<T, V, NA><<<unsigned(ndof), nt, 0, st>>>(static_cast<const T*>(f), Nv, c0, cw, U)
+#define GO(T, V) row_moments_kernel<T, V, NA><<<unsigned(ndof), kRowSlots, 0, st>>>(static_cast<const T*>(f), Nv, c0, cw, U)
     if (fp64) {
         if (v4) GO(double, 4);
         else GO(double, 1);

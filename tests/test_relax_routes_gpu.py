@@ -85,3 +85,34 @@ def test_ars_and_bdf_routes(cuda, name, Nv, dtype):
             per_q[q].append(torch.cat([Fq[0][:5].double().flatten(), new[:5].flatten()]))
     for outs in per_stage + list(per_q.values()):
         _agree(outs, dtype)
+
+
+@pytest.mark.parametrize('name', ['bgk-direct-gll', 'esbgk-direct-gll', 'shakov-direct-gll'])
+@pytest.mark.parametrize('Nv,dtype', [(24, torch.float32), (16, torch.float64), (10, torch.float32)])
+def test_row_count_does_not_change_a_bit(cuda, name, Nv, dtype):
+    """A row's moments, stage and BDF step have the same bits in a list of any
+    length (a partitioned run is the serial one): every thread count of the
+    kernels."""
+    from frfs_b200.integrators import STEPPERS
+    vm, sm = _model(name, Nv, dtype)
+    f = _rows(vm, 3, 5, dtype)
+    L = [0.2 * (a - b) for a, b in zip(f, f[1:] + f[:1])]
+    A, B = STEPPERS['adgfs-ars-443'], STEPPERS['adgfs-bdf-2']
+    outs = []
+    for n in (5, 591, 592, 1500):
+        F, Ls = [_place(x, n, 0) for x in f], [_place(x, n, 0) for x in L]
+        mom = lambda: torch.zeros(n, sm.nalph, dtype=torch.float64, device='cuda')
+        U, LU = [mom() for _ in range(4)], [mom() for _ in range(3)]
+        got = []
+        for ar in (1, 2, 3):
+            out = torch.empty_like(F[0])
+            sm.ars_stage(n, 0.01, ar, 2 | 4 | 8 | (1 if ar == 1 else 0), A._A_expl(ar), A._A_impl(ar), F[:ar], out,
+                         Ls[:ar], U[:ar + 1], LU[:ar])
+            got.append(out)
+        Uq, LUq, new = [mom() for _ in range(2)], [mom() for _ in range(2)], mom()
+        sm.bdf_step(n, 0.01, 1, 1, [0.0, 1.0], [0.0], 0.0, [F[0]], F[0], [Ls[0]], [Uq[0]], [LUq[0]], mom())
+        out = torch.empty_like(F[0])
+        sm.bdf_step(n, 0.01, 2, 7, B.bdf_A, [-x for x in B.bdf_G], B.bdf_B, F[:2], out, Ls[:2], Uq, LUq, new)
+        outs.append([x[:5].clone() for x in got + [out, new] + U + LU + Uq + LUq])
+    for o in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(o, outs[0]))
