@@ -540,18 +540,24 @@ __global__ void __launch_bounds__(128, (NU <= 16 && sizeof(T) == 4) ? 4 : 3) rhs
 
 // uf: face-value rows [E][NF]; or, with fsel, the solution-point rows of u
 // ([E][NU]) read at row fsel[f] (GATHER, M0 rows unit vectors).
-// One CTA per wall face point.  Bound by latency: few CTAs, two rows each.  So
-// a thread has two chunks of both rows in flight, its velocity index moves by
-// carries, the normal is padded to three components, and meshes with few wall
-// points get 1024 threads a row (bc_update_threads).  24^3 FP32 on one B200: 1926
-// points 76 -> 34 us, 256 points 16.7 -> 6.3 us, 84 points 14.1 -> 5.3 us.
-template <typename T>
-__global__ void __launch_bounds__(1024) bc_update_kernel(const bdgfs_fr_eles el,
-                                                         const bdgfs_fr_walls wl,
-                                                         const T* __restrict__ uf,
-                                                         const int32_t* __restrict__ fsel)
+// One CTA of NT threads per wall face point.  Bound by latency: few CTAs, two rows
+// each.  So a thread has two or four chunks of both rows in flight, its velocity
+// index moves by carries, the normal is padded to three components, and meshes with
+// few wall points get 512 threads a row (bc_update_launch).  A point's two sums are
+// made of kWallSlots partial sums each with either NT: a mesh in parts, with fewer
+// wall points each, gives the bits of the whole.  Within 1 % (3 % on 60 points) of the
+// form whose sums followed 256, 512 or 1024 threads, which took 34, 6.3 and 5.3 us for
+// 1926, 256 and 84 points of 24^3 FP32 on one B200 (76, 16.7, 14.1 with one chunk in
+// flight).
+constexpr int kWallSlots = 512;
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) bc_update_kernel(const bdgfs_fr_eles el, const bdgfs_fr_walls wl,
+                                                       const T* __restrict__ uf, const int32_t* __restrict__ fsel)
 {
-    __shared__ double red[2 * 32];
+    constexpr int G = kWallSlots / NT;
+    static_assert(kWallSlots == 16 * 32 && kWallSlots % NT == 0, "slots and warps");
+    __shared__ double red[2][kWallSlots / 32];
     __shared__ T cs[1024];                                    // cell-centre velocities (Nv <= 1024)
     const int w = blockIdx.x;
     const int e = wl.fpt[2 * w], f = wl.fpt[2 * w + 1];
@@ -577,63 +583,87 @@ __global__ void __launch_bounds__(1024) bc_update_kernel(const bdgfs_fr_eles el,
     const T* __restrict__ ul = fsel ? uf + (int64_t(e) * el.nupts + fsel[f]) * el.nv
                                     : uf + (int64_t(e) * el.nfpts + f) * el.nv;
     const T* c0 = static_cast<const T*>(el.c0);
-    for (int i = threadIdx.x; i < Nv; i += blockDim.x) cs[i] = c0[i];
+    for (int i = threadIdx.x; i < Nv; i += NT) cs[i] = c0[i];
     __syncthreads();
-    double s0 = 0.0, s1 = 0.0;
-    auto add = [&](T fac, T a, T b) {
-        if (fac >= T(0)) s0 += double(fac * a);
-        else s1 += double(fac * b);
+    double s0[G], s1[G];                                      // partial sums threadIdx.x + g NT
+#pragma unroll
+    for (int g = 0; g < G; ++g) s0[g] = s1[g] = 0.0;
+    auto add = [&](int g, T fac, T a, T b) {
+        if (fac >= T(0)) s0[g] += double(fac * a);
+        else s1[g] += double(fac * b);
     };
     // four velocities of one z line per step (16-byte loads) when rows are
     // aligned and 4 divides Nv
     const bool v4 = Nv % 4 == 0 && (reinterpret_cast<uintptr_t>(ul) & 15u) == 0 &&
                     (reinterpret_cast<uintptr_t>(fw) & 15u) == 0;
     if (v4) {
-        const uint32_t n = uint32_t(el.nv), st = blockDim.x * 4;
+        constexpr uint32_t st = NT * 4;
+        constexpr int U = NT == 512 ? 4 : 2;                  // chunks in flight
+        const uint32_t n = uint32_t(el.nv);
         RowWalk x(threadIdx.x * 4, st, uint32_t(Nv));
-        auto step = [&](const Chunk<T, 4>& a, const Chunk<T, 4>& b) {
-            const T f0 = (cs[x.ix] - uw[0]) * pn[0], f1 = (cs[x.iy] - uw[1]) * pn[1];
+        for (uint32_t v = threadIdx.x * 4; v < n; v += U * st) {
+            Chunk<T, 4> a[U], b[U];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) add(f0 + f1 + (cs[x.iz + q] - uw[2]) * pn[2], a.v[q], b.v[q]);
-            x.next();
-        };
-        for (uint32_t v = threadIdx.x * 4; v < n; v += 2 * st) {
-            Chunk<T, 4> a[2], b[2];
-            a[0].load(ul + v);
-            b[0].load(fw + v);
-            const bool two = v + st < n;
-            if (two) {
-                a[1].load(ul + v + st);
-                b[1].load(fw + v + st);
+            for (int k = 0; k < U; ++k) {
+                if (v + k * st < n) {
+                    a[k].load(ul + v + k * st);
+                    b[k].load(fw + v + k * st);
+                }
             }
-            step(a[0], b[0]);
-            if (two) step(a[1], b[1]);
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                if (v + k * st < n) {
+                    const T f0 = (cs[x.ix] - uw[0]) * pn[0], f1 = (cs[x.iy] - uw[1]) * pn[1];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        add(k % G, f0 + f1 + (cs[x.iz + q] - uw[2]) * pn[2], a[k].v[q], b[k].v[q]);
+                }
+                x.next();
+            }
         }
     } else {
-        for (int64_t v = threadIdx.x; v < el.nv; v += blockDim.x) {
-            T c[3];
-            vel(cs, Nv, v, c);
-            add((c[0] - uw[0]) * pn[0] + (c[1] - uw[1]) * pn[1] + (c[2] - uw[2]) * pn[2], ul[v], fw[v]);
+        for (int64_t v0 = threadIdx.x; v0 < el.nv; v0 += kWallSlots) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int64_t v = v0 + g * NT;
+                if (v < el.nv) {
+                    T c[3];
+                    vel(cs, Nv, v, c);
+                    add(g, (c[0] - uw[0]) * pn[0] + (c[1] - uw[1]) * pn[1] + (c[2] - uw[2]) * pn[2], ul[v], fw[v]);
+                }
+            }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        for (int o = 16; o > 0; o >>= 1) {
+            s0[g] += __shfl_xor_sync(0xffffffffu, s0[g], o);
+            s1[g] += __shfl_xor_sync(0xffffffffu, s1[g], o);
+        }
+        if (lane == 0) {
+            red[0][(threadIdx.x + g * NT) / 32] = s0[g];
+            red[1][(threadIdx.x + g * NT) / 32] = s1[g];
+        }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { red[2 * warp] = s0; red[2 * warp + 1] = s1; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a0 = 0.0, a1 = 0.0;
-        for (int i = 0; i < int(blockDim.x >> 5); ++i) { a0 += red[2 * i]; a1 += red[2 * i + 1]; }
-        T* out = static_cast<T*>(wl.bcv);
-        out[2 * w] = T(a0 * wl.cw);
-        out[2 * w + 1] = T(a1 * wl.cw);
+    if (threadIdx.x < 32) {                                   // lanes 0..15: the first sum, 16..31: the second
+        double s = red[lane >> 4][lane & 15];
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((lane & 15) == 0) static_cast<T*>(wl.bcv)[2 * w + (lane >> 4)] = T(s * wl.cw);
     }
 }
 
-// threads per wall point: 1024 while two such CTAs per SM hold every point
-static unsigned bc_update_threads(int nwall) { return nwall <= 148 * 2 ? 1024 : nwall <= 148 * 4 ? 512 : 256; }
+// 512 threads per wall point while four such CTAs per SM hold every point, else 256
+template <typename T>
+static int bc_update_launch(const bdgfs_fr_eles& el, const bdgfs_fr_walls& wl, const void* uf, const int32_t* fsel,
+                            cudaStream_t st)
+{
+    const T* p = static_cast<const T*>(uf);
+    if (wl.nwall <= 148 * 4) bc_update_kernel<T, 512><<<wl.nwall, 512, 0, st>>>(el, wl, p, fsel);
+    else bc_update_kernel<T, 256><<<wl.nwall, 256, 0, st>>>(el, wl, p, fsel);
+    return cuda_status(cudaGetLastError());
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) residual_kernel(const T* __restrict__ a,
@@ -833,13 +863,8 @@ extern "C" int32_t bdgfs_fr_bc_update(const bdgfs_fr_eles* el, const bdgfs_fr_wa
     if (wl->nwall < 0 || !wl->fpt || !wl->bcid || !wl->uwall || !wl->fw || !wl->bcv)
         return BDGFS_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (el->fp64)
-        bc_update_kernel<double><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const double*>(uf),
-                                                            nullptr);
-    else
-        bc_update_kernel<float><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const float*>(uf),
-                                                           nullptr);
-    return cuda_status(cudaGetLastError());
+    return el->fp64 ? bc_update_launch<double>(*el, *wl, uf, nullptr, st)
+                    : bc_update_launch<float>(*el, *wl, uf, nullptr, st);
 }
 
 extern "C" int32_t bdgfs_fr_bc_update_gather(const bdgfs_fr_eles* el, const bdgfs_fr_walls* wl,
@@ -852,11 +877,7 @@ extern "C" int32_t bdgfs_fr_bc_update_gather(const bdgfs_fr_eles* el, const bdgf
     if (wl->nwall < 0 || !wl->fpt || !wl->bcid || !wl->uwall || !wl->fw || !wl->bcv)
         return BDGFS_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (el->fp64)
-        bc_update_kernel<double><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const double*>(u), fsel);
-    else
-        bc_update_kernel<float><<<wl->nwall, bc_update_threads(wl->nwall), 0, st>>>(*el, *wl, static_cast<const float*>(u), fsel);
-    return cuda_status(cudaGetLastError());
+    return el->fp64 ? bc_update_launch<double>(*el, *wl, u, fsel, st) : bc_update_launch<float>(*el, *wl, u, fsel, st);
 }
 
 extern "C" int32_t bdgfs_fr_rhs(const bdgfs_fr_eles* el, const bdgfs_fr_walls* wl, const void* u,

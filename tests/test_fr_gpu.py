@@ -161,6 +161,57 @@ def test_partitioned_virtual_ranks_equal_single_domain(cuda):
                            s.eles_scal_upts_inb_full[0].index_select(0, idx)), r
 
 
+@pytest.mark.parametrize('prec', ['single', 'double'])
+@pytest.mark.parametrize('shift', [0, 1])
+def test_wall_sums_do_not_depend_on_the_number_of_walls(cuda, prec, shift):
+    """A wall point's sums have the same bits in a launch over any number of wall
+    points (a part of a mesh has fewer than the whole): every thread count of
+    the kernel, rows on and off a 16-byte boundary."""
+    from frfs_b200 import _lib
+    cfg, be, mesh, s = _system('quad', 3, prec, Nv=16, Nrho=4, M=6, dev=5, shape=(90, 2))
+    _perturb(s, 3)
+    src = s.eles_scal_upts_inb_full[0]
+    u = torch.empty(src.numel() + shift, dtype=src.dtype, device=src.device)[shift:].view(src.shape).copy_(src)
+    total = s.walls.nwall
+    assert total > 2 * 297
+    got = {}
+    for nw in (1, 296, 297, 592, 593, total):
+        wl = _lib.FrWall.from_buffer_copy(s.walls.struct)
+        wl.nwall = nw
+        s.walls.bcv.fill_(float('nan'))
+        _lib.check(_lib.lib().bdgfs_fr_bc_update_gather(_lib.ref(s.ele.struct), _lib.ref(wl),
+                                                        s.ele.fsel.data_ptr(), u.data_ptr(), _lib.stream_ptr()),
+                   'bdgfs_fr_bc_update_gather')
+        got[nw] = s.walls.bcv[:nw].clone()
+    assert bool(torch.isfinite(got[total]).all())
+    for nw, b in got.items():
+        assert torch.equal(b, got[total][:nw]), nw
+
+
+def test_partition_with_many_walls_equals_single_domain(cuda):
+    """The same as above with more wall points than one launch shape covers:
+    whole mesh and parts run the wall update with different thread counts."""
+    from frfs_b200.partition import LocalTransport, slab_partition, step_rk2_virtual
+    cfg, be, mesh, s = _system('quad', 3, 'single', Nv=16, Nrho=4, M=6, dev=5, shape=(90, 2))
+    _perturb(s, 4)
+    parts = slab_partition(mesh, 3)
+    systems = [DGFSSystem(be, mesh, cfg, nreg=3, partition=(parts, r)) for r in range(3)]
+    assert s.walls.nwall > 592 and max(sy.walls.nwall for sy in systems) <= 296
+    tr = LocalTransport(systems)
+    for r, sy in enumerate(systems):
+        sy.transport = tr
+        idx = torch.as_tensor(parts[r], device=be.device)
+        sy.eles_scal_upts_inb_full[0].copy_(s.eles_scal_upts_inb_full[0].index_select(0, idx))
+    integ = get_integrator(be, s, cfg)
+    integ.use_graph = False
+    for _ in range(2):
+        integ.step(0.0, 5e-4)
+        step_rk2_virtual(systems, 5e-4)
+    for r, sy in enumerate(systems):
+        idx = torch.as_tensor(parts[r], device=be.device)
+        assert torch.equal(sy.eles_scal_upts_inb_full[0], s.eles_scal_upts_inb_full[0].index_select(0, idx)), r
+
+
 @pytest.mark.parametrize('kind,order', [('quad', 3), ('hex', 2), ('quad', 2)])
 def test_tensor_core_rhs_matches_cuda_core_rhs(cuda, kind, order):
     """The tcgen05 (3xTF32) FR residual against the CUDA-core kernel on the
