@@ -43,14 +43,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase)
 // arrival; with arrive = 0 nothing arrives, so the wait runs out after
 // `limit` polls and the status word gets BDGFS_ETIMEOUT (no copy or MMA is
 // in flight, no TMEM is held); with arrive = 1 the thread arrives first and
-// the wait succeeds (BDGFS_OK).
+// the wait succeeds (BDGFS_OK).  Both kinds of wait, which must agree.
 __global__ void wait_probe_kernel(uint32_t limit, int arrive, int32_t* status)
 {
     __shared__ __align__(8) uint64_t bar;
+    __shared__ int lost;
     if (threadIdx.x != 0) return;
+    lost = 0;
     mbar_init(&bar, 1);
     if (arrive) mbar_arrive(&bar);
-    *status = mbar_wait_bounded(&bar, 0, limit) ? BDGFS_OK : BDGFS_ETIMEOUT;
+    const bool done = mbar_wait_bounded(&bar, 0, limit);
+    mbar_wait_or_lose(&bar, 0, &lost, limit);
+    const bool marked = isnan(lost_nan(&lost, 1.f));
+    if (marked) mbar_wait_or_lose(&bar, 0, &lost);      // returns at once: the CTA waits no more
+    *status = done == marked ? BDGFS_EINVAL : done ? BDGFS_OK : BDGFS_ETIMEOUT;
 }
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)

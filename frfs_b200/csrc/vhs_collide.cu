@@ -697,7 +697,7 @@ __device__ __forceinline__ void p2_pass1_spectrum_tm(int tr, const float4* ez, f
 // DFT of a warp overlap the other warps' loads instead of waiting at a CTA
 // barrier; two CTA barriers per transform remain (z stored, y stored).
 // wfree: that mbarrier (NT arrivals per phase), wpar: this thread's phase
-// parity, counter: the work counter, whose bit 62 a timed-out wait sets.
+// parity, lost: the CTA's flag of a wait that ran out.
 // BAL (with SPLIT, 320 threads): in the transform loop warps 0-7 carry the
 // pencil pairs 0..255 on f32x2 arithmetic and warps 8-9 the remaining 32
 // pairs as 64 single pencils on scalar arithmetic (thread 256 + 2e + s:
@@ -710,7 +710,7 @@ template <bool SPLIT, bool BAL = false, bool FHT = false>
 __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict__ f,
                                float* __restrict__ Qout, double* mom, int flags,
                                unsigned char* smem, unsigned char* scratch, uint32_t tmem,
-                               uint64_t* wfree, uint32_t& wpar, unsigned long long* counter)
+                               uint64_t* wfree, uint32_t& wpar, volatile int* lost)
 {
     using namespace p2;
     const int project = flags & BDGFS_PROJECT;
@@ -889,15 +889,9 @@ __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict_
                 }
             };
             // every thread's x-pass loads done: W is free (bounded wait; on
-            // expiry bit 62 of the work counter ends the launch)
+            // expiry the CTA gives NaN)
             auto wait_free = [&]() {
-                uint32_t spins = 0;
-                while (!tc::mbar_try(wfree, wpar)) {
-                    if (++spins == (1u << 22)) {
-                        atomicOr(counter, 1ull << 62);
-                        break;
-                    }
-                }
+                tc::mbar_wait_or_lose(wfree, wpar, lost);
                 wpar ^= 1u;
             };
             if constexpr (FHT) {
@@ -1223,6 +1217,7 @@ __device__ void collide_one_p2(const bdgfs_vhs_grid& g, const float* __restrict_
         float2 vr[N], vi[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) { vr[i] = ld2(Wr + i * PS + y * RS + z); vi[i] = ld2(Wi + i * PS + y * RS + z); }
+        vr[0] = f2(tc::lost_nan(lost, vr[0].x), tc::lost_nan(lost, vr[0].y));
         dft_p2<N, +1>(vr, vi);
         const double cy = need_m ? g.c0[y] : 0.0;
         const double cz0 = need_m ? g.c0[z] : 0.0, cz1 = need_m ? g.c0[z + 1] : 0.0;
@@ -1330,11 +1325,15 @@ __global__ void __launch_bounds__(NT, 1) __maxnreg__(65536 / NT / 8 * 8 > 255 ? 
     __shared__ int64_t s_start[5];
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_wfree;
+    __shared__ volatile int s_lost;
     constexpr bool kPacked = V0::pk || V1::pk;
     constexpr uint32_t kTmemCols = (V0::fht || V1::fht) ? 2 * p2::TMEM_COLS : p2::TMEM_COLS;
     if constexpr (kPacked) {
         if (threadIdx.x < 32) tc::tmem_alloc(&s_tmem, kTmemCols);
-        if (threadIdx.x == 0) tc::mbar_init(&s_wfree, NT);
+        if (threadIdx.x == 0) {
+            tc::mbar_init(&s_wfree, NT);
+            s_lost = 0;
+        }
         tc::tc_fence_before();
     }
     uint32_t wpar = 0;
@@ -1378,7 +1377,7 @@ __global__ void __launch_bounds__(NT, 1) __maxnreg__(65536 / NT / 8 * 8 > 255 ? 
         if (g.Nv == V0::n) {
             if constexpr (V0::pk)
                 collide_one_p2<V0::split, V0::bal, V0::fht>(g, f, Q, mom, a.flags, smem, scratch, tmem, &s_wfree, wpar,
-                                          a.counter);
+                                          &s_lost);
             else
                 collide_one<T, V0::n, NT, V0::wg, V0::sg, V0::gr, V0::sl>(
                     g, f, Q, mom, a.flags, smem, scratch);
@@ -1386,7 +1385,7 @@ __global__ void __launch_bounds__(NT, 1) __maxnreg__(65536 / NT / 8 * 8 > 255 ? 
             if (g.Nv == V1::n) {
                 if constexpr (V1::pk)
                     collide_one_p2<V1::split, V1::bal, V1::fht>(g, f, Q, mom, a.flags, smem, scratch, tmem, &s_wfree,
-                                              wpar, a.counter);
+                                              wpar, &s_lost);
                 else
                     collide_one<T, V1::n, NT, V1::wg, V1::sg, V1::gr, V1::sl>(
                         g, f, Q, mom, a.flags, smem, scratch);

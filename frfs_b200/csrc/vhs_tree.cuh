@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
     __shared__ int64_t s_start[5];
     __shared__ SplitPlan s_plan;
     __shared__ int s_last;
+    __shared__ volatile int s_lost;
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_free;
     __shared__ TreePlan pl;
@@ -185,7 +186,10 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
     const int project = a.flags & BDGFS_PROJECT;
 
     if (tid < 32) tc::tmem_alloc(&s_tmem, kCols);
-    if (tid == 0) tc::mbar_init(&s_free, NT);
+    if (tid == 0) {
+        tc::mbar_init(&s_free, NT);
+        s_lost = 0;
+    }
     tc::tc_fence_before();
     for (int i = tid; i < 3 * M; i += NT) {
         const cpx<float> v = phase[i * N + 1], w = phase[size_t(Nrho - 1) * M * 3 * N + i * N + 1];
@@ -222,17 +226,11 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
     const bool two = tid + NT < NZ;
 
     // Exchange round: wait until every thread has read the last one's
-    // elements, store, barrier, load, arrive.  The wait is bounded; on expiry
-    // bit 62 of the work counter ends the launch.
+    // elements, store, barrier, load, arrive.  The wait is bounded; on expiry the
+    // CTA gives NaN.
     uint32_t par = 1;
     auto wait_free = [&]() {
-        uint32_t spins = 0;
-        while (!tc::mbar_try(&s_free, par)) {
-            if (++spins == (1u << 22)) {
-                atomicOr(a.counter, 1ull << 62);
-                break;
-            }
-        }
+        tc::mbar_wait_or_lose(&s_free, par, &s_lost);
         par ^= 1u;
         __syncwarp();
     };
@@ -557,6 +555,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
         if (ns > 1) {
             // the part that arrives last adds the radii in order and finishes the
             // distribution
+            if (s_lost) G[-N * NT].x = tc::lost_nan(&s_lost, 0.f);
             __threadfence();
             __syncthreads();
             if (tid == 0) s_last = atomicAdd(a.tickets + it.cut, 1u) == uint32_t(ns - 1);
@@ -625,6 +624,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
                 }
             }
             if (r) arrive();
+            vr[0].x = tc::lost_nan(&s_lost, vr[0].x);
             dft_p2<N, +1>(vr, vi);
             load_row(f + (r ? row1 : row0), fvec, S[r]);
             double q0 = 0.0, q1 = 0.0, q2 = 0.0;

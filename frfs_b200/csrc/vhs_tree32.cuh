@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
     __shared__ int64_t s_start[5];
     __shared__ SplitPlan s_plan;
     __shared__ int s_last;
+    __shared__ volatile int s_lost;
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_free;
     __shared__ TreePlan pl;
@@ -96,7 +97,10 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
     auto kz_of = [&](int r) { return r == 2 ? H : warp + 8 * r; };
 
     if (tid < 32) tc::tmem_alloc(&s_tmem, 512);
-    if (tid == 0) tc::mbar_init(&s_free, NT);
+    if (tid == 0) {
+        tc::mbar_init(&s_free, NT);
+        s_lost = 0;
+    }
     tc::tc_fence_before();
     for (int i = tid; i < 3 * M; i += NT) {
         const cpx<float> v = phase[i * N + 1], w = phase[size_t(Nrho - 1) * M * 3 * N + i * N + 1];
@@ -122,13 +126,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
 
     uint32_t par = 1;
     auto wait_free = [&]() {
-        uint32_t spins = 0;
-        while (!tc::mbar_try(&s_free, par)) {
-            if (++spins == (1u << 22)) {
-                atomicOr(a.counter, 1ull << 62);
-                break;
-            }
-        }
+        tc::mbar_wait_or_lose(&s_free, par, &s_lost);
         par ^= 1u;
         __syncwarp();
     };
@@ -515,6 +513,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
         if (ns > 1) {
             // the part that arrives last adds the radii in order and finishes the
             // distribution
+            if (s_lost) G[warp * N - N * ROW].x = tc::lost_nan(&s_lost, 0.f);
             __threadfence();
             __syncthreads();
             if (tid == 0) s_last = atomicAdd(a.tickets + it.cut, 1u) == uint32_t(ns - 1);
@@ -630,6 +629,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
                 }
             }
             if (j == 3) arrive();
+            vr[0].x = tc::lost_nan(&s_lost, vr[0].x);
             dft_p2<N, +1>(vr, vi);
             float u[N];
             load_row(f + row_at(j), fvec, u);

@@ -50,7 +50,6 @@ struct VssPairArgs {
     unsigned char* slots;            // [cut distribution][radius] kSlot
     uint32_t* tickets;               // [cut distribution], zeroed
     SplitPlan plan;
-    uint32_t* timeout;               // set when a bounded wait ran out
 };
 
 __device__ __forceinline__ float2 v2(float a, float b) { return make_float2(a, b); }
@@ -113,12 +112,19 @@ __device__ __noinline__ void vssp_merge(const float4* from, float4* to, int Nrho
     }
 }
 
+// NaN in place of what a CTA gives of which a wait ran out
+__device__ __noinline__ void vssp_lose(float* p, int n)
+{
+    for (int i = 0; i < n; ++i) p[i] = __int_as_float(0x7fffffff);
+}
+
 __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs a)
 {
     using namespace vssp;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_tmem;
     __shared__ int s_last;
+    __shared__ volatile int s_lost;
     __shared__ __align__(8) uint64_t s_free;
     const bdgfs_vss_pair_args& g = a.g;
     float4* W = reinterpret_cast<float4*>(smem);
@@ -126,7 +132,10 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
     float4* E = W + N * PX;                                    // [axis][k]: (E1.re, E2.re, E1.im, E2.im)
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid < 32) tc::tmem_alloc(&s_tmem, 512);
-    if (tid == 0) tc::mbar_init(&s_free, NT);
+    if (tid == 0) {
+        tc::mbar_init(&s_free, NT);
+        s_lost = 0;
+    }
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
@@ -136,14 +145,8 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
     const uint32_t tcol = s_tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(2 * kTask * (warp >> 2));
 
     uint32_t par = 1;
-    bool dead = false;                                          // a wait ran out: finish without waiting again
-    auto wait_free = [&]() {
-        for (uint32_t spins = 0; !dead && !tc::mbar_try(&s_free, par);) {
-            if (++spins == (1u << 22)) {
-                dead = true;
-                atomicOr(a.timeout, 1u);
-            }
-        }
+    auto wait_free = [&]() {                                    // bounded; on expiry the CTA gives NaN
+        tc::mbar_wait_or_lose(&s_free, par, &s_lost);
         par ^= 1u;
         __syncwarp();
     };
@@ -388,6 +391,7 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
         }
 
         if (ns > 1) {
+            if (s_lost) vssp_lose(reinterpret_cast<float*>(Gs + size_t(it.b0) * N * NZ + tid), 4);
             __threadfence();
             __syncthreads();
             if (tid == 0) s_last = atomicAdd(a.tickets + it.cut, 1u) == uint32_t(ns - 1);
@@ -439,6 +443,7 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
                 dft_p2<N, +1>(vr, vi);
 #pragma unroll
                 for (int z = 0; z < N; ++z) Q[t * N + z] = vr[z].x - fp[t * N + z] * vr[z].y;
+                if (s_lost) vssp_lose(Q + t * N, N);
             }
         }
     }
@@ -455,7 +460,7 @@ __global__ void __launch_bounds__(vssp::NT, 1) vss_pair_kernel(const VssPairArgs
 
 using namespace bdgfs;
 
-// scratch: [timeout word, tickets, padding][F per CTA][slots]
+// scratch: [tickets, padding][F per CTA][sum per CTA][slots]
 static size_t vssp_head(int64_t nslots) { return (size_t(nslots + 1) * sizeof(uint32_t) + 255) / 256 * 256; }
 
 extern "C" int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas)
@@ -488,14 +493,13 @@ extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* sc
     VssPairArgs a{};
     a.g = *g;
     a.plan = split_plan(g->ndof, nslots, g->Nrho, int(nctas), 0.3f, 0.4f);
-    a.timeout = reinterpret_cast<uint32_t*>(base);
-    a.tickets = a.timeout + 1;
+    a.tickets = reinterpret_cast<uint32_t*>(base);
     a.F = reinterpret_cast<unsigned char*>(base + vssp_head(nslots));
     a.sums = a.F + size_t(nctas) * kF;
     a.slots = a.sums + size_t(nctas) * kSlot;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(a.timeout, 0, sizeof(uint32_t) * (1 + size_t(g->ndof - a.plan.whole)), st) != cudaSuccess)
-        return BDGFS_ECUDA;
+    const size_t cut = size_t(g->ndof - a.plan.whole);
+    if (cut > 0 && cudaMemsetAsync(a.tickets, 0, sizeof(uint32_t) * cut, st) != cudaSuccess) return BDGFS_ECUDA;
     if (const int rc = smem_optin(reinterpret_cast<const void*>(vss_pair_kernel), kSmem)) return rc;
     nctas = std::min(nctas, split_items(g->ndof, a.plan));
     vss_pair_kernel<<<unsigned(nctas), NT, kSmem, st>>>(a);

@@ -215,3 +215,19 @@ def test_inifile_accessors():
     assert c.getfloat('a', 'missing', 3.0) == 3.0
     assert c.getexpr('a', 'b', subs=c.items('constants')) == '(24*2.5)'
     assert c.items_as('constants', float) == {'Nv': 24.0, 'x0': 2.5}
+
+
+def test_exchange_waits_that_run_out_are_marked():
+    """The kernels whose threads wait for each other's reads of an exchange
+    buffer poll in one place only, which marks the CTA on expiry, and each of
+    them stores NaN for a marked CTA (the state check finds it)."""
+    import glob
+    import frfs_b200
+    csrc = os.path.join(os.path.dirname(frfs_b200.__file__), 'csrc')
+    text = {os.path.basename(f): open(f).read() for f in glob.glob(csrc + '/*.cu*')}
+    # the GEMM-shaped kernels report BDGFS_ETIMEOUT through their status word
+    polls = {f for f, t in text.items() if 'mbar_try(' in t}
+    assert polls == {'tcgen05.cuh', 'tc_gemm_tma.cu', 'fr_tc.cu'}
+    waits = {f for f, t in text.items() if 'mbar_wait_or_lose(' in t} - {'tcgen05.cuh', 'tc_gemm.cu'}
+    assert waits == {'vhs_collide.cu', 'vhs_tree.cuh', 'vhs_tree32.cuh', 'vss_pair.cu'}
+    assert all('lost_nan(' in text[f] or 'vssp_lose(' in text[f] for f in waits)
