@@ -36,6 +36,20 @@ __host__ __device__ inline SplitPlan split_plan(int64_t total, int64_t nslots, i
     return SplitPlan{best > 1 ? total - tail : total, best};
 }
 
+// What a launch passes to its kernel: the plan where the host knows the list's length,
+// else (ns = 0) what the kernel plans with once it has read the counts.
+struct SplitArgs {
+    SplitPlan plan;
+    int64_t nslots;                 // slots of cut items' blocks, after one per CTA
+    int32_t nctas;                  // CTAs that a full round has
+    float once, again;
+};
+
+__device__ __forceinline__ SplitPlan split_plan(const SplitArgs& s, int64_t total, int nb)
+{
+    return s.plan.ns > 0 ? s.plan : split_plan(total, s.nslots, nb, s.nctas, s.once, s.again);
+}
+
 // Work item -> position in the list, its blocks [b0, b1) of nb, parts of it, and
 // its place among the cut items
 struct SplitItem {

@@ -1615,8 +1615,9 @@ static int launch(const bdgfs_vhs_grid* grids, int ngrids, const bdgfs_vhs_batch
 
 // Arguments and grid of a kernel that cuts short lists over radii: the scratch
 // holds tickets, and per CTA ``priv`` bytes and a slot (G^), then as many slots for
-// the radii of cut distributions as fit; the plan is made in the kernel (a batch's
-// count may be on the device), and here for the grid.  Clears the counter and the tickets; *nblk = 0: nothing to do.
+// the radii of cut distributions as fit; the plan is made here, or in the kernel where a
+// batch's count is on the device.  Clears the counter and the tickets; *nblk = 0: nothing
+// to do.
 template <typename Args>
 static int split_launch(Args& a, const bdgfs_vhs_grid* grids, const bdgfs_vhs_batch* batches, int nbatch, int flags,
                         void* scratch, size_t scratch_bytes, uint64_t* counter, size_t priv, size_t slot, int ctas_per_sm,
@@ -1645,15 +1646,15 @@ static int split_launch(Args& a, const bdgfs_vhs_grid* grids, const bdgfs_vhs_ba
     if (ctas < 1) return BDGFS_ESCRATCH;
     // tickets, private parts, a slot per CTA, slots of cut distributions
     const size_t head = (size_t(ctas) * sizeof(uint32_t) + 255) / 256 * 256, used = head + size_t(ctas) * (priv + slot);
-    a.nctas = int32_t(ctas);
     a.tickets = reinterpret_cast<uint32_t*>(base);
     unsigned char* at = reinterpret_cast<unsigned char*>(base + head);
     a.slots = at + size_t(ctas) * priv;
     *private_at = at;
-    a.nslots = room > used ? int64_t((room - used) / slot) : 0;
-    SplitPlan plan{total, 1};
-    if (!dev_count) plan = split_plan(total, a.nslots, a.g.Nrho, int(ctas), once, again);
-    const int64_t cut = dev_count ? std::min(total, ctas) : total - plan.whole;     // one ticket each
+    a.split = SplitArgs{{0, 0}, room > used ? int64_t((room - used) / slot) : 0, int32_t(ctas), once, again};
+    SplitPlan& plan = a.split.plan;
+    if (!dev_count) plan = split_plan(total, a.split.nslots, a.g.Nrho, int(ctas), once, again);
+    // one ticket each: never more than a round of CTAs
+    const int64_t cut = dev_count ? std::min(total, ctas) : total - plan.whole;
     if (cut > 0 && cudaMemsetAsync(a.tickets, 0, size_t(cut) * sizeof(uint32_t), st) != cudaSuccess)
         return BDGFS_ECUDA;
     if (cudaMemsetAsync(counter, 0, sizeof(uint64_t), st) != cudaSuccess) return BDGFS_ECUDA;

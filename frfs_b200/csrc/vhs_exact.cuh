@@ -58,8 +58,7 @@ struct ExactArgs {
     int32_t nbatch, flags;
     unsigned char* slots;
     uint32_t* tickets;
-    int64_t nslots;                 // slots of cut distributions' radii, after one per CTA
-    int32_t nctas;                  // CTAs that a full round has
+    SplitArgs split;                // slots: radii of cut distributions, after one per CTA
     unsigned long long* counter;
 };
 
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(Exact<T, N>::NT) vhs_exact_kernel(const ExactA
             }
             s_start[b + 1] = s_start[b] + c;
         }
-        s_plan = split_plan(s_start[a.nbatch], a.nslots, Nrho, a.nctas, 0.5f, 0.6f);
+        s_plan = split_plan(a.split, s_start[a.nbatch], Nrho);
     }
     __syncthreads();
     // pencil of every pass; threads beyond N^2 (Nv = 12) take no part
@@ -303,7 +302,7 @@ __global__ void __launch_bounds__(Exact<T, N>::NT) vhs_exact_kernel(const ExactA
             forward_yz();
             if (tid < NH * N) {
                 const T* gwp = gw + size_t(p) * N * NH * N + tid;
-                cpx<T>* to = (ns > 1 ? slot_at(a.nctas + it.cut * Nrho + p) : G) + tid;
+                cpx<T>* to = (ns > 1 ? slot_at(a.split.nctas + it.cut * Nrho + p) : G) + tid;
                 const bool acc = ns == 1 && p > 0;
 #pragma unroll
                 for (int kz = 0; kz < N; ++kz) {
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(Exact<T, N>::NT) vhs_exact_kernel(const ExactA
                 for (int kz = 0; kz < N; ++kz) s[kz] = {T(0), T(0)};
 #pragma unroll 1
                 for (int j = 0; j < Nrho; ++j) {
-                    const T* src = reinterpret_cast<const T*>(slot_at(a.nctas + it.cut * Nrho + j) + tid);
+                    const T* src = reinterpret_cast<const T*>(slot_at(a.split.nctas + it.cut * Nrho + j) + tid);
 #pragma unroll
                     for (int kz = 0; kz < N; ++kz) {
                         s[kz].x = add_rn(s[kz].x, __ldcg(src + 2 * kz * NH * N));

@@ -98,8 +98,7 @@ struct TreeArgs {
     int32_t nbatch, flags;
     unsigned char* slots;
     uint32_t* tickets;              // one per cut distribution, zeroed before the launch
-    int64_t nslots;                 // slots of cut distributions' radii, after one per CTA
-    int32_t nctas;                  // CTAs that a full round has
+    SplitArgs split;                // slots: radii of cut distributions, after one per CTA
     unsigned long long* counter;
 };
 
@@ -205,7 +204,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
             }
             s_start[b + 1] = s_start[b] + c;
         }
-        s_plan = split_plan(s_start[a.nbatch], a.nslots, Nrho, a.nctas, 1.5f, 1.7f);
+        s_plan = split_plan(a.split, s_start[a.nbatch], Nrho);
     }
     __syncthreads();
     tc::tc_fence_after();
@@ -347,7 +346,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
         }
 
         // G^ of this thread, [kx * NT]: the sum so far, or one slot per radius (cut)
-        const int64_t slot = ns > 1 ? a.nctas + it.cut * Nrho + it.b0 : int64_t(blockIdx.x);
+        const int64_t slot = ns > 1 ? a.split.nctas + it.cut * Nrho + it.b0 : int64_t(blockIdx.x);
         float2* G = reinterpret_cast<float2*>(a.slots + size_t(slot) * QLayoutTree::slot_bytes()) + tid;
         for (int p = it.b0; p < it.b1; ++p) {
             // ---- node factors of radius p ----
@@ -562,7 +561,7 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
-            const float2* Gj = reinterpret_cast<const float2*>(a.slots + size_t(a.nctas + it.cut * Nrho) * QLayoutTree::slot_bytes()) + tid;
+            const float2* Gj = reinterpret_cast<const float2*>(a.slots + size_t(a.split.nctas + it.cut * Nrho) * QLayoutTree::slot_bytes()) + tid;
 #pragma unroll
             for (int k = 0; k < N; ++k) vr[k].x = vi[k].x = 0.f;
 #pragma unroll 1

@@ -53,8 +53,7 @@ struct Tree32Args {
     unsigned char* priv;
     unsigned char* slots;
     uint32_t* tickets;
-    int64_t nslots;                 // slots of cut distributions' radii, after one per CTA
-    int32_t nctas;
+    SplitArgs split;                // slots: radii of cut distributions, after one per CTA
     unsigned long long* counter;
 };
 
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
             }
             s_start[b + 1] = s_start[b] + c;
         }
-        s_plan = split_plan(s_start[a.nbatch], a.nslots, Nrho, a.nctas, 1.5f, 1.7f);
+        s_plan = split_plan(a.split, s_start[a.nbatch], Nrho);
     }
     __syncthreads();
     tc::tc_fence_after();
@@ -294,7 +293,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
         }
 
         // G^ [kx][kz][ky]: the sum so far, or one slot per radius (cut)
-        const int64_t slot = ns > 1 ? a.nctas + it.cut * Nrho + it.b0 : int64_t(blockIdx.x);
+        const int64_t slot = ns > 1 ? a.split.nctas + it.cut * Nrho + it.b0 : int64_t(blockIdx.x);
         float2* G = reinterpret_cast<float2*>(a.slots + size_t(slot) * QLayoutTree32::slot_bytes()) + lane;
         for (int p = it.b0; p < it.b1; ++p) {
             const cpx<float>* php = phase + size_t(p) * M * 3 * N;
@@ -520,7 +519,7 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
             __syncthreads();
             if (!s_last) continue;
             __threadfence();
-            G0 = reinterpret_cast<const float2*>(a.slots + size_t(a.nctas + it.cut * Nrho) * QLayoutTree32::slot_bytes()) + lane;
+            G0 = reinterpret_cast<const float2*>(a.slots + size_t(a.split.nctas + it.cut * Nrho) * QLayoutTree32::slot_bytes()) + lane;
         }
 
         // ---- lane A: QG = IFFT(G^), lane B: fC = IFFT(bb2 F) ----
