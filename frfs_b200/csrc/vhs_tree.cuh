@@ -184,12 +184,10 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
     const float* bb2 = static_cast<const float*>(g.bb2);
     const int project = a.flags & BDGFS_PROJECT;
 
-    if (tid < 32) tc::tmem_alloc(&s_tmem, kCols);
     if (tid == 0) {
         tc::mbar_init(&s_free, NT);
         s_lost = 0;
     }
-    tc::tc_fence_before();
     for (int i = tid; i < 3 * M; i += NT) {
         const cpx<float> v = phase[i * N + 1], w = phase[size_t(Nrho - 1) * M * 3 * N + i * N + 1];
         buf[i] = make_float4(v.x, v.y, w.x, w.y);
@@ -207,9 +205,14 @@ __global__ void __launch_bounds__(tree::NT, 1) vhs_tree_kernel(const TreeArgs a)
         s_plan = split_plan(a.split, s_start[a.nbatch], Nrho);
     }
     __syncthreads();
-    tc::tc_fence_after();
-    if (tid == 0) tree_plan(phase, Nrho, M, pl, buf);
+    // nothing to do (a device count of zero): leave before the tree and tensor memory
+    // (18.5 -> 7.3 us with the launch's two memsets, one B200)
+    if (s_start[a.nbatch] == 0) return;
+    if (tid < 32) tc::tmem_alloc(&s_tmem, kCols);
+    tc::tc_fence_before();
+    if (tid == 32) tree_plan(phase, Nrho, M, pl, buf);
     __syncthreads();
+    tc::tc_fence_after();
     const uint32_t lane0 = s_tmem + (uint32_t(32 * (warp & 3)) << 16);
     const uint32_t tab = lane0 + kAB + uint32_t(4 * N * (warp >> 2));
     const uint32_t tsp = lane0 + kS + uint32_t(2 * N * (warp >> 2));     // S_p of z-pencil 0; + N: of 1

@@ -95,12 +95,10 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
     const int ntask = warp == 0 ? 3 : 2;                           // kz of the x- and y-passes
     auto kz_of = [&](int r) { return r == 2 ? H : warp + 8 * r; };
 
-    if (tid < 32) tc::tmem_alloc(&s_tmem, 512);
     if (tid == 0) {
         tc::mbar_init(&s_free, NT);
         s_lost = 0;
     }
-    tc::tc_fence_before();
     for (int i = tid; i < 3 * M; i += NT) {
         const cpx<float> v = phase[i * N + 1], w = phase[size_t(Nrho - 1) * M * 3 * N + i * N + 1];
         buf[i] = make_float4(v.x, v.y, w.x, w.y);
@@ -118,9 +116,14 @@ __global__ void __launch_bounds__(tree32::NT, 1) vhs_tree32_kernel(const Tree32A
         s_plan = split_plan(a.split, s_start[a.nbatch], Nrho);
     }
     __syncthreads();
-    tc::tc_fence_after();
-    if (tid == 0) tree_plan(phase, Nrho, M, pl, buf);
+    // nothing to do (a device count of zero): leave before the tree and tensor memory
+    // (18.5 -> 7.3 us with the launch's two memsets, one B200)
+    if (s_start[a.nbatch] == 0) return;
+    if (tid < 32) tc::tmem_alloc(&s_tmem, 512);
+    tc::tc_fence_before();
+    if (tid == 32) tree_plan(phase, Nrho, M, pl, buf);
     __syncthreads();
+    tc::tc_fence_after();
     const uint32_t tab = s_tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(256 * (warp >> 2));   // + 128 r
 
     uint32_t par = 1;

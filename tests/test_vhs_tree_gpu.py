@@ -16,13 +16,14 @@ from helpers import mixed_maxwellians, oracle_for, rel_l2, vhs_cfg
 pytestmark = pytest.mark.gpu
 
 TREE = 10                               # tile index among the 24^3 FP32 variants
+TILES = {24: TREE, 32: 3}
 
 
-def _setup(Nrho, M, ssrule=None):
+def _setup(Nrho, M, ssrule=None, Nv=24):
     from frfs_b200.backend import CUDABackend
     from frfs_b200.scattering import DGFSVHSGLLScatteringModel
     from frfs_b200.velocitymesh import DGFSVelocityMesh
-    cfg = vhs_cfg(24, Nrho, M, 6, extra=f'tile = {TREE}')
+    cfg = vhs_cfg(Nv, Nrho, M, 6, extra=f'tile = {TILES[Nv]}')
     if ssrule:
         cfg.set('spherical-design-rule', 'ssrule', str(ssrule))
     be = CUDABackend(cfg)
@@ -157,3 +158,41 @@ def test_scratch_limits(cuda):
     assert call(per) == 0
     assert float((q - want).norm() / want.norm()) < 2e-5
     assert call(1024) == -5
+
+
+@pytest.mark.parametrize('Nv,old,new', [(24, 9, TREE), (32, 2, 3)])
+def test_a_launch_with_nothing_to_do_is_short(cuda, Nv, old, new):
+    """A device list whose count is zero (the fallback list of every hybrid call)
+    costs no more than twice what the variants without a direction tree take for
+    it: the kernel leaves before it builds the tree.  Device time of launches in
+    a graph."""
+    from frfs_b200.scattering import VHSCollider
+    be, vm, sm = _setup(12, 12, Nv=Nv)
+    f = torch.zeros(64, Nv**3, device=cuda)
+    q = torch.full_like(f, 7.0)
+    idx = torch.zeros(64, dtype=torch.int32, device=cuda)
+    cnt = torch.zeros(1, dtype=torch.int64, device=cuda)
+
+    def per_launch(tile):
+        sm.grid.struct.tile = tile
+        col = VHSCollider([sm.grid], be.device)
+        run = lambda: col([(0, f, q, None)], index=idx, count=cnt)
+        run()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(50):
+                run()
+        best = 1e30
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.replay()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 20.0)
+        return best
+    t_old, t_new = per_launch(old), per_launch(new)
+    print(f'{Nv}^3: empty launch {t_old:.2f} us, with a tree {t_new:.2f} us')
+    assert t_new < 2 * t_old
+    assert bool((q == 7.0).all())
