@@ -28,7 +28,7 @@ EXPORTS = (
     'bdgfs_bgk_moments', 'bdgfs_bgk_maxwellian', 'bdgfs_ars_stage',
     'bdgfs_esbgk_moments', 'bdgfs_esbgk_gaussian', 'bdgfs_shakov_moments', 'bdgfs_shakov_target',
     'bdgfs_bdf_step', 'bdgfs_vss_scratch_bytes', 'bdgfs_vss_collide', 'bdgfs_vss_project',
-    'bdgfs_vss_pair_scratch_bytes', 'bdgfs_vss_pair_collide',
+    'bdgfs_vss_pair_scratch_bytes', 'bdgfs_vss_pair_scratch_for', 'bdgfs_vss_pair_collide',
 )
 
 
@@ -222,6 +222,8 @@ def lib():
             fn.argtypes = at
         L.bdgfs_vss_pair_scratch_bytes.restype = C.c_int64
         L.bdgfs_vss_pair_scratch_bytes.argtypes = [C.c_int32]
+        L.bdgfs_vss_pair_scratch_for.restype = C.c_int64
+        L.bdgfs_vss_pair_scratch_for.argtypes = [C.c_int32, C.c_int64, C.c_int32]
         _lib = L
     return _lib
 

@@ -470,6 +470,16 @@ extern "C" int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas)
     return int64_t(vssp_head(7 * int64_t(nctas)) + size_t(nctas) * (vssp::kF + 8 * vssp::kSlot) + 256);
 }
 
+extern "C" int64_t bdgfs_vss_pair_scratch_for(int32_t nctas, int64_t ndof, int32_t Nrho)
+{
+    if (nctas < 1 || ndof < 1 || Nrho < 1) return 0;
+    // CTAs with work, and the slots of the last round's distributions where those of
+    // nctas CTAs are enough to cut it
+    const int64_t ctas = ndof >= nctas ? nctas : std::min<int64_t>(nctas, ndof * Nrho);
+    const int64_t cut = ndof % ctas * Nrho, nslots = cut <= 7 * int64_t(nctas) ? cut : 0;
+    return int64_t(vssp_head(nslots) + size_t(ctas) * (vssp::kF + vssp::kSlot) + size_t(nslots) * vssp::kSlot + 256);
+}
+
 extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* scratch, int64_t bytes, void* stream)
 {
     using namespace vssp;
@@ -484,7 +494,8 @@ extern "C" int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* g, void* sc
     // CTAs and slots that fit
     const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
     const int64_t room = bytes - int64_t(base - reinterpret_cast<uintptr_t>(scratch));
-    int64_t nctas = std::min<int64_t>(nsm, (room - int64_t(vssp_head(0))) / int64_t(kF + kSlot));
+    const int64_t work = g->ndof >= nsm ? nsm : std::min<int64_t>(nsm, g->ndof * g->Nrho);
+    int64_t nctas = std::min<int64_t>(work, (room - int64_t(vssp_head(0))) / int64_t(kF + kSlot));
     if (nctas < 1) return BDGFS_ESCRATCH;
     int64_t nslots = 0;
     while (int64_t(vssp_head(nslots + 1) + size_t(nctas) * (kF + kSlot) + size_t(nslots + 1) * kSlot) <= room &&

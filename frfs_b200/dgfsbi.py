@@ -281,7 +281,7 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
                              bcross=t['bcross'].data_ptr(), c=t['c'].data_ptr())
         for p in (0, 1):
             a.f[p], a.Q[p] = fs[p].data_ptr(), Qs[p].data_ptr()
-        nb = L.bdgfs_vss_pair_scratch_bytes(self._nctas)
+        nb = L.bdgfs_vss_pair_scratch_for(self._nctas, ndof, self.vm.Nrho())
         if self._scratch is None or self._scratch.numel() < nb:
             self._scratch = torch.empty(nb, dtype=torch.uint8, device=self.backend.device)
         _lib.check(L.bdgfs_vss_pair_collide(C.byref(a), self._scratch.data_ptr(), nb, _lib.stream_ptr()),

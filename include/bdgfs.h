@@ -596,6 +596,10 @@ typedef struct bdgfs_vss_pair_args {
 /* Bytes of device scratch for nctas CTAs (one per SM runs every launch at full
  * speed; less runs fewer CTAs, below one CTA's BDGFS_ESCRATCH). */
 int64_t bdgfs_vss_pair_scratch_bytes(int32_t nctas);
+/* Bytes with which a call of ndof distributions runs as with those (0: an
+ * argument below 1): a pair of distributions needs 8 MB instead of the 295 MB
+ * of 148 CTAs. */
+int64_t bdgfs_vss_pair_scratch_for(int32_t nctas, int64_t ndof, int32_t Nrho);
 int32_t bdgfs_vss_pair_collide(const bdgfs_vss_pair_args* a, void* scratch,
                                int64_t bytes, void* stream);
 

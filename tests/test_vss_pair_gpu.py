@@ -146,3 +146,33 @@ def test_pair_scratch_limits(cuda):
     assert call(s.numel()) == -1
     a.M, a.Nv = 2, 16
     assert call(s.numel()) == -3
+
+
+def test_pair_scratch_follows_the_call(cuda):
+    """A model holds what its largest call needs (a slot is 24 24^2 float4s: 221
+    KB; a CTA has two, a radius of a cut distribution one), and a call in the
+    least scratch gives the bits of a call in the most."""
+    from frfs_b200 import _lib
+    be, vm, sm = _model(6, 6)
+    L, slot = _lib.lib(), 24**3 * 16
+    most = L.bdgfs_vss_pair_scratch_bytes(sm._nctas)
+    base = _rows(vm, 4)
+    held = 0
+    for n, slots in ((1, 6 * 2 + 6), (5, 30 * 2 + 30), (20, 120 * 2 + 120), (3, 0), (150, 148 * 2 + 12)):
+        pick = torch.arange(n) % 4
+        fs = [f[pick].contiguous() for f in base]
+        Q, W = [[torch.full_like(f, float('nan')) for f in fs] for _ in range(2)]
+        sm.collide(fs, Q)
+        if sm._nctas == 148:
+            held = max(held, slots * slot)
+            assert held <= sm._scratch.numel() <= held + 8192
+        keep, sm._scratch = sm._scratch, torch.empty(most, dtype=torch.uint8, device='cuda')
+        a = _lib.VssPairArgs(Nv=24, Nrho=6, M=6, ndof=n, phase=sm._pair['phase'].data_ptr(),
+                             bself=sm._pair['bself'].data_ptr(), bcross=sm._pair['bcross'].data_ptr(),
+                             c=sm._pair['c'].data_ptr())
+        for p in (0, 1):
+            a.f[p], a.Q[p] = fs[p].data_ptr(), W[p].data_ptr()
+        _lib.check(L.bdgfs_vss_pair_collide(_lib.ref(a), sm._scratch.data_ptr(), most, _lib.stream_ptr()), 'pair')
+        sm._scratch = keep
+        assert all(torch.equal(q, w) for q, w in zip(Q, W))
+    assert [L.bdgfs_vss_pair_scratch_for(*a) for a in ((0, 1, 1), (1, 0, 1), (1, 1, 0))] == [0, 0, 0]
