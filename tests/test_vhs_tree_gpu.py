@@ -1,12 +1,12 @@
-"""The shift-tree form of the 24^3 FP32 collision kernel: direction sets with
-every kind of tree node, work split over radii, ragged lists, and rows that
+"""The shift-tree form of the 24^3 and 32^3 FP32 collision kernels: direction sets
+with every kind of tree node, work split over radii, ragged lists, and rows that
 are not 16-byte aligned.
 
 Reference: the FP64 oracle (<= 1e-3 of Q and 1e-5 of the loss term, the bounds
-of the other FP32 variants), and between two runs of the kernel that differ
-only in how radii are split over CTAs, 2e-5 of Q: the partial sums of the gain
-are associated differently, and Q's gain-loss cancellation turns 1e-7 of the
-terms into about 1e-5 of Q."""
+of the other FP32 variants).  A distribution has the same bits whole or cut over
+radii, wherever it stands in a list, however many CTAs run, on and off a 16-byte
+boundary and in place: runs that differ in these only are compared with
+torch.equal."""
 import numpy as np
 import pytest
 import torch
@@ -34,6 +34,9 @@ def _setup(Nrho, M, ssrule=None, Nv=24):
 def _rows(vm, n, seed=5):
     rng = np.random.default_rng(seed)
     return torch.from_numpy(np.stack([mixed_maxwellians(vm.cv(), rng) for _ in range(n)])).float().cuda()
+
+
+grids = pytest.mark.parametrize('Nv', [24, 32])
 
 
 def _check(vm, f, q, rows):
@@ -65,43 +68,48 @@ DESIGNS = {
 }
 
 
+@grids
 @pytest.mark.parametrize('name', list(DESIGNS))
-def test_direction_trees(cuda, tmp_path, name):
+def test_direction_trees(cuda, tmp_path, name, Nv):
     half = DESIGNS[name]
-    be, vm, sm = _setup(4, len(half), _design(tmp_path, half))
+    be, vm, sm = _setup(4 if Nv == 24 else 2, len(half), _design(tmp_path, half), Nv)
     f = _rows(vm, 2)
     q = torch.full_like(f, float('nan'))
     sm.collide(f, q, project=False)
     _check(vm, f, q, (0, 1))
 
 
-def test_too_many_directions_has_no_tree(cuda, tmp_path):
+@grids
+def test_too_many_directions_has_no_tree(cuda, tmp_path, Nv):
     from frfs_b200.autotune import variants
     half = np.random.default_rng(1).normal(size=(49, 3))
     cfg_path = _design(tmp_path, half)
-    be, vm, sm48 = _setup(2, 12)
+    be, vm, sm48 = _setup(2, 12, Nv=Nv)
     from frfs_b200.scattering import VHSGrid
     sz = np.loadtxt(cfg_path)[:49]
-    g = VHSGrid(24, vm.L(), vm.qz(), vm.qw(), sz, vm.sw(), 0.38, 1.0, vm.cw(), vm.c0(), torch.float32, be.device)
+    g = VHSGrid(Nv, vm.L(), vm.qz(), vm.qw(), sz, vm.sw(), 0.38, 1.0, vm.cw(), vm.c0(), torch.float32, be.device)
     assert len(variants([g])) == len(variants([sm48.grid])) - 1
 
 
+@grids
 @pytest.mark.parametrize('M', [12, 6])
 @pytest.mark.parametrize('n', [1, 13, 75, 149, 297])
-def test_split_over_radii_agrees(cuda, M, n):
-    """Short lists cut the radii into parts (1 row: one part per radius; the
-    others fewer, or none); 600 rows are not cut."""
-    be, vm, sm = _setup(12, M)
+def test_split_over_radii_agrees(cuda, M, n, Nv):
+    """Short lists and the last round of long ones cut the radii into parts (1
+    row: one part per radius; others fewer, or none).  Of 600 rows, 592 are whole
+    on 148 SMs and 8 are cut: every row has the bits of the short list."""
+    be, vm, sm = _setup(12 if Nv == 24 else 5, M, Nv=Nv)
     f = _rows(vm, 8)[torch.arange(n) % 8].contiguous()
     q = torch.full_like(f, float('nan'))
     mom = torch.full((n, 10), float('nan'), dtype=torch.float64, device=f.device)
     sm.collide(f, q, moments=mom)
-    big = f[torch.arange(600) % n].contiguous()
+    rows = torch.arange(600) % n
+    big = f[rows].contiguous()
     qb = torch.empty_like(big)
     sm.collide(big, qb)
-    assert float((q - qb[:n]).double().norm() / qb[:n].double().norm()) < 2e-5
+    assert torch.equal(qb, q[rows])
     assert torch.isfinite(mom).all() and float(mom[:, 5:].abs().max()) < 1e-12
-    # the same launch again: bitwise (the parts are added in order)
+    # the same launch again
     q2 = torch.empty_like(q)
     sm.collide(f, q2)
     assert torch.equal(q, q2)
@@ -110,11 +118,12 @@ def test_split_over_radii_agrees(cuda, M, n):
         _check(vm, f, q, (0,))
 
 
-def test_device_list_and_unaligned_rows(cuda):
+@grids
+def test_device_list_and_unaligned_rows(cuda, Nv):
     """A device index list with a device count (the split follows the count),
     entries out of range skipped; rows at a 4-byte offset; in place."""
-    be, vm, sm = _setup(12, 12)
-    n3 = 24**3
+    be, vm, sm = _setup(12 if Nv == 24 else 5, 12, Nv=Nv)
+    n3 = Nv**3
     f = _rows(vm, 8)[torch.arange(40) % 8].contiguous()
     want = torch.empty_like(f)
     sm.collide(f, want)
@@ -126,7 +135,7 @@ def test_device_list_and_unaligned_rows(cuda):
         done = [i for i in idx[:count].tolist() if 0 <= i < 40]
         for i in range(40):
             if i in done:
-                assert float((q[i] - want[i]).norm() / want[i].norm()) < 2e-5
+                assert torch.equal(q[i], want[i])
             else:
                 assert not bool(q[i].any())
     g = torch.empty(3 * n3 + 1, device=f.device)[1:].view(3, n3)
@@ -134,17 +143,18 @@ def test_device_list_and_unaligned_rows(cuda):
     q = torch.empty(3 * n3 + 1, device=f.device)[1:].view(3, n3)
     assert g.data_ptr() % 16 == 4
     sm.collide(g, q)
-    assert float((q - want[:3]).norm() / want[:3].norm()) < 2e-5
+    assert torch.equal(q, want[:3])
     h = f[:3].clone()
     sm.collide(h, h)
-    assert float((h - want[:3]).norm() / want[:3].norm()) < 2e-5
+    assert torch.equal(h, want[:3])
 
 
-def test_scratch_limits(cuda):
+@grids
+def test_scratch_limits(cuda, Nv):
     """One CTA's scratch is enough; less than a slot is refused."""
     import ctypes as C
     from frfs_b200 import _lib
-    be, vm, sm = _setup(12, 12)
+    be, vm, sm = _setup(12 if Nv == 24 else 5, 12, Nv=Nv)
     f = _rows(vm, 5)
     want, q = torch.empty_like(f), torch.full_like(f, float('nan'))
     sm.collide(f, want)
@@ -156,7 +166,7 @@ def test_scratch_limits(cuda):
     call = lambda n: _lib.lib().bdgfs_vhs_collide(arr, 1, bs, 1, 1, s.data_ptr(), C.c_size_t(n),
                                                   counter.data_ptr(), _lib.stream_ptr())
     assert call(per) == 0
-    assert float((q - want).norm() / want.norm()) < 2e-5
+    assert torch.equal(q, want)
     assert call(1024) == -5
 
 
