@@ -1562,7 +1562,8 @@ static int choose(const bdgfs_vhs_grid* grids, int ngrids)
         if (grids[i].fp64 != grids[0].fp64) return -1;
         if (grids[i].Nrho < 1 || grids[i].M < 1 || grids[i].M > 64) return -1;
     }
-    int tile = grids[0].tile, k = 0;
+    const int tile = grids[0].tile == BDGFS_TILE_BY_GRID ? 0 : grids[0].tile;
+    int k = 0;
     for (int i = 0; i < kNumEntries; ++i) {
         if (!entry_matches(kEntries[i], grids, ngrids)) continue;
         if (k == tile) return i;

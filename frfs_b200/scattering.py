@@ -116,7 +116,7 @@ class VHSGrid:
 
 
 # tile value of a grid set that ``autotune.tune_vhs`` found faster as one launch
-# per grid (no tile index of bdgfs_vhs_tiles)
+# per grid (BDGFS_TILE_BY_GRID: the C entry points themselves run it as tile 0)
 BY_GRID = -1
 
 

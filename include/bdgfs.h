@@ -29,6 +29,11 @@ extern "C" {
  * Fast-spectral VHS collision operator Q(f, f)
  * ---------------------------------------------------------------------- */
 
+/* Tile of grids for which a tuner found one launch per grid faster than one
+ * over the set: a caller that splits its batches by grid acts on it, the entry
+ * points take the set in one launch as with tile 0. */
+#define BDGFS_TILE_BY_GRID (-1)
+
 /* One velocity grid (Nv^3 cube) with its precomputed tables.  All table
  * pointers are device pointers; "real" means float when fp64 == 0 and
  * double when fp64 == 1, "complex" the matching (re, im) pair. */
@@ -38,7 +43,8 @@ typedef struct bdgfs_vhs_grid {
     int32_t M;           /* half-sphere directions                          */
     int32_t fp64;        /* 0: FP32 state/tables, 1: FP64                   */
     int32_t tile;        /* kernel variant (threads per CTA), 0 = default;
-                            see bdgfs_vhs_tiles                             */
+                            see bdgfs_vhs_tiles; BDGFS_TILE_BY_GRID runs
+                            as 0                                            */
     int32_t pad_;
     double prefac;       /* VHS prefactor                                   */
     double cw;           /* velocity cell volume (2L/Nv)^3                  */

@@ -99,3 +99,36 @@ def test_bad_lists_are_refused_before_any_launch(cuda, by_grid):
             col(batches)
     torch.cuda.synchronize()
     assert all(bool((x == 7.0).all()) for x in q)
+
+
+def test_c_entry_points_take_a_set_tuned_by_grid(cuda):
+    """Grids that the tuner marked BY_GRID are still a valid argument of the C
+    entry points: one launch, as with tile 0."""
+    from frfs_b200 import _lib
+    from frfs_b200.scattering import BY_GRID
+    grids, fs = _grids()
+    L, out = _lib.lib(), []
+    for tile in (0, BY_GRID):
+        for g in grids:
+            g.struct.tile = tile
+        arr = (_lib.VhsGrid * 2)(*[g.struct for g in grids])
+        nb = L.bdgfs_vhs_scratch_bytes(arr, 2, 0)
+        assert nb > 0
+        scratch = torch.empty(nb, dtype=torch.uint8, device=cuda)
+        counter = torch.zeros(1, dtype=torch.int64, device=cuda)
+        for static in (False, True):
+            q = [torch.full_like(f, float('nan')) for f in fs]
+            bs = (_lib.VhsBatch * 2)(*[_lib.VhsBatch(grid=i, ndof=6, f=fs[i].data_ptr(), Q=q[i].data_ptr())
+                                       for i in (0, 1)])
+            if static:
+                rc = L.bdgfs_vhs_collide_static(arr, 2, bs, 2, 1, _lib.stream_ptr())
+            else:
+                rc = L.bdgfs_vhs_collide(arr, 2, bs, 2, 1, _lib.ptr(scratch), nb, _lib.ptr(counter),
+                                         _lib.stream_ptr())
+            assert rc == 0
+            torch.cuda.synchronize()
+            out.append(q)
+    for q in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(q, out[0]))
+    arr[0].tile = -2
+    assert L.bdgfs_vhs_scratch_bytes(arr, 2, 0) == 0
