@@ -97,10 +97,39 @@ def q_flops_per_eval(Nv, Nrho, M):
     return (M * Nrho + Nrho + 2) * 5.0 * n * math.log2(n) + 8.0 * M * Nrho * n
 
 
+def direction_tree(sz):
+    """Nodes (x, y, leaves) of the shift tree of directions sz: distinct |s_x|, s_y
+    below an x-node, |s_z| below a y-node, with opposite directions the same."""
+    nodes = [set(), set(), set()]
+    for s in sz:
+        s = [round(float(c), 9) + 0.0 for c in s]
+        if next((c for c in s if c != 0.0), 0.0) < 0.0:
+            s = [-c + 0.0 for c in s]
+        nodes[0].add(s[0])
+        nodes[1].add((s[0], s[1]))
+        nodes[2].add((s[0], s[1], abs(s[2])))
+    return tuple(len(n) for n in nodes)
+
+
+def q_flops_shift_tree(Nv, Nrho, nodes):
+    """FLOP of one evaluation by the shift-tree kernels (csrc/vhs_tree.cuh):
+    1-D FFTs at 5 N log2 N, two lanes a line.  Per radius 2 N (N/2 + 1) lines a
+    node of the x- and y-passes, 2 N^2 a leaf, and the forward transform of a real
+    cube; 12 and 8 FLOP per value for the shifts and the products.  Around the
+    radii, the forward transform of f and the pair of inverse ones."""
+    import math
+    nx, ny, nl = nodes
+    half, line = Nv * (Nv // 2 + 1), 5.0 * Nv * math.log2(Nv)
+    forward = Nv**2 / 2 + 2 * half
+    per_radius = (2 * half * (nx + ny) + 2 * Nv**2 * nl + forward) * line \
+        + 12.0 * Nv * half * (nx + ny) + 8.0 * Nv**3 * nl
+    return Nrho * per_radius + (forward + 4 * half + 2 * Nv**2) * line
+
+
 def q_flops_reference_equivalent(Nv, Nrho, M):
     """FLOP of the reference's own evaluation of one Q (scattering.py:
     239-281): 3 M Nrho + 3 complex FFTs at 5 n log2 n, n = Nv^3.  Reported
-    beside the roofline only as context; the roofline uses the packed count."""
+    beside the roofline only as context; the roofline counts the kernel's own."""
     import math
     n = Nv**3
     return (3 * M * Nrho + 3) * 5.0 * n * math.log2(n)
@@ -464,10 +493,11 @@ def config_block(n):
 
 # ---------------------------------------------------------------- other configs
 BATCHED = dict(n24=24576, n32=8192, Nrho=16, M=12, dev=6, omega=0.81, mass2=2.0)
-# DRAM bytes (read + write) of one collision launch on the 2048-DOF Couette
-# state, from an ncu capture of the tuner's Nv=24 variant (the balanced
-# packed variant with the z-pass spectra in tensor memory: 114.2 MB + 93.5 MB)
-Q_LAUNCH_DRAM_BYTES = 114.22e6 + 93.46e6
+# tile of the shift-tree kernel among the Nv=24 FP32 variants; DRAM bytes (read +
+# write) of one launch on 2048 distributions from ncu captures of it and of the
+# variant with the z-pass spectra in tensor memory
+Q_TREE_TILE = 10
+Q_TREE_DRAM_BYTES, Q_PACKED_DRAM_BYTES = 113.88e6 + 78.56e6, 114.22e6 + 93.46e6
 SMALL64 = dict(Nv=16, Nrho=8, M=6, dev=5, omega=0.5, order=2, nx=4, ny=4, dt=1e-3)
 
 
@@ -548,7 +578,8 @@ def batched_q(flush, reps=3, sizes=None):
         cons[f'Nv{g.Nv}'] = q_conservation(lambda f2, q2, m, gi=gi: col([(gi, f2, q2, m)]),
                                            fs[gi], qs[gi], g.c0.double(), float(g.struct.cw))
     return {'workload': f"two species, {w['n24']} x 24^3 + {w['n32']} x 32^3, mass ratio 2, Nrho=16, M=12, "
-                        'one persistent launch in a CUDA graph, FP32 + FP64 projection',
+                        + ('one persistent launch per grid' if grids[0].struct.tile < 0 else
+                           'one persistent launch') + ' in a CUDA graph, FP32 + FP64 projection',
             'q_evals_per_s': ndof / (t * 1e-3), 'ms_per_launch': t,
             'tiles': [int(x.struct.tile) for x in grids], 'conservation': cons}, (grids, fs, qs)
 
@@ -739,8 +770,12 @@ def vss_mixture(flush, peak=None, reps=3, ndof=None, check=True):
         tot += a.elapsed_time(b)
     ms = tot / reps
     P = vm.Nrho() * vm.M()
-    flop_item = (S * (3 * P + 1) + 2) * 5 * n * math.log2(n) + 38 * S * P * n
-    flop = flop_item * S * nd
+    if sm._pair is not None:
+        # opposite directions share slices: 2 P of them for both gains, three transforms
+        # each, and three a species around them
+        flop = nd * ((6 * P + 6) * 5 * n * math.log2(n) + 38 * 2 * P * n)
+    else:
+        flop = nd * S * ((S * (3 * P + 1) + 2) * 5 * n * math.log2(n) + 38 * S * P * n)
     res = {'workload': (f"binary gas mixture (molar masses {w['masses'][0]}, {w['masses'][1]} kg/mol), "
                         f"'vss-gll' alpha={w['alpha']} omega={w['omega']}, Nv={w['Nv']}^3 on "
                         f"[-{w['dev']},{w['dev']}]^3, Nrho={w['Nrho']}, M={w['M']} full-sphere "
@@ -1311,7 +1346,10 @@ def run_gpu(args):
         qt.append((a, b))
     torch.cuda.synchronize()
     q_ms = sum(x.elapsed_time(y) for x, y in qt) / len(qt)
-    flop = q_flops_per_eval(WORK['Nv'], WORK['Nrho'], WORK['M']) * ndof
+    tree = system.sm.grid.struct.tile == Q_TREE_TILE
+    flop = ndof * (q_flops_shift_tree(WORK['Nv'], WORK['Nrho'], direction_tree(system.vm.sz())) if tree else
+                   q_flops_per_eval(WORK['Nv'], WORK['Nrho'], WORK['M']))
+    packed = ndof * q_flops_per_eval(WORK['Nv'], WORK['Nrho'], WORK['M'])
     achieved = flop / (q_ms * 1e-3) / 1e12
     # measured FP32 FMA peak on this GPU (probe kernel in libbdgfs)
     probe = torch.zeros(1, device=dev)
@@ -1433,23 +1471,30 @@ def run_gpu(args):
         'data': 'synthetic', 'config': config_block(ws),
         'q_evals_per_s': ws * 2 * ndof * args.steps / t_max,
         'q_rel_l2_err_vs_fp64_reference': qerr,
-        'roofline': {'bound': 'fp32', 'kernel': 'bdgfs::vhs_collide_kernel',
+        'roofline': {'bound': 'fp32',
+                     'kernel': 'bdgfs::vhs_tree_kernel' if tree else 'bdgfs::vhs_collide_kernel',
                      'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s',
                      'frac': achieved / peak,
                      'peak_source': 'measured FP32 FMA probe on this GPU (MEASURED_PEAKS.json has '
                                     'no FP32 CUDA-core figure)',
                      'flop_per_launch': flop, 'launch_ms': q_ms,
+                     'packed_equivalent': {
+                         'flop_per_launch': packed, 'tflops': packed / (q_ms * 1e-3) / 1e12,
+                         'note': ('one complex FFT per direction and radius in the same launch time; '
+                                  'context only (the shift tree does about 0.6 of it)')},
                      'reference_equivalent': {
                          'flop_per_launch': ndof * q_flops_reference_equivalent(24, 12, 12),
                          'tflops': ndof * q_flops_reference_equivalent(24, 12, 12) / (q_ms * 1e-3) / 1e12,
                          'note': ("the reference's 3 M Nrho + 3 FFTs per Q in the same launch time; "
-                                  'context only (above the peak: the packed algorithm does fewer)')},
+                                  'context only (above the peak: the kernel does fewer)')},
                      # algorithmic: f in + Q out = 2 x 113 MB
-                     'traffic': Q_LAUNCH_DRAM_BYTES, 'traffic_alg': 2 * 4 * ndof * 24**3,
+                     'traffic': Q_TREE_DRAM_BYTES if tree else Q_PACKED_DRAM_BYTES,
+                     'traffic_alg': 2 * 4 * ndof * 24**3,
                      'traffic_source': ('not measured in this run: dram__bytes_read.sum + '
                                         'dram__bytes_write.sum of one ncu capture of this '
-                                        'kernel variant on the same 2048 Couette cubes '
-                                        '(profiles/vhs_collide_nv24.md)')},
+                                        'kernel on 2048 distributions ('
+                                        + ('profiles/kernel_counters.md)' if tree else
+                                           'profiles/vhs_collide_nv24.md)'))},
         'e2e': {'value': e2e, 'unit': 'DG steps/s', 'h2d_bytes_per_step': nbytes,
                 'd2h_bytes_per_step': nbytes},
         'gpu_launches': launches,

@@ -23,6 +23,19 @@ def test_flop_models():
     assert bench.q_flops_reference_equivalent(24, 12, 12) > 2.4 * bench.q_flops_per_eval(24, 12, 12)
 
 
+def test_shift_tree_flop_model():
+    """Mirrored and opposite directions share nodes, directions without common
+    components share none.  By hand at 24^3: 312 lines a half pass, 576 a full one."""
+    shared = [(1.0, 0.5, 0.3), (1.0, 0.5, -0.3), (-1.0, -0.5, 0.3), (0.0, 0.0, 1.0), (0.0, 0.0, -1.0)]
+    assert bench.direction_tree(shared) == (2, 2, 2)
+    assert bench.direction_tree([(0.1, 0.2, 0.3), (0.4, 0.5, 0.6)]) == (2, 2, 2)
+    line = 5 * 24 * math.log2(24)
+    radius = (2 * 312 * 8 + 2 * 576 * 6 + 288 + 624) * line + 12 * 24 * 312 * 8 + 8 * 13824 * 6
+    ends = (288 + 624 + 4 * 312 + 2 * 576) * line
+    assert bench.q_flops_shift_tree(24, 12, (2, 6, 6)) == pytest.approx(12 * radius + ends)
+    assert 0.6 < bench.q_flops_shift_tree(24, 12, (2, 6, 6)) / bench.q_flops_per_eval(24, 12, 12) < 0.65
+
+
 def test_config_block_names_the_workload():
     one, four = bench.config_block(1), bench.config_block(4)
     for c in (one, four):
