@@ -374,8 +374,9 @@ __device__ __forceinline__ double target_at(const Target& t, const double (*ex)[
 // AR > 0: the stage at compile time, so that a thread has all 2 AR rows of a
 // chunk (of two chunks for AR <= 2) in flight at once; AR = 0 reads the stage
 // from the arguments.  The moment algebra (pow, divisions) runs in one warp, a
-// lane per implicit stage, instead of in every thread.  Bound: HBM; the FP64
-// pipe and the conversions are about half of it.
+// lane per implicit stage, instead of in every thread.  Bound: the
+// latency of HBM loads (0.65 of the copy rate at 28 warps an SM; conversions 29 %,
+// FP64 20 %).
 template <typename T, int VEC, int NA, int AR>
 __global__ void __launch_bounds__(512, NA == 5 && AR <= 2 ? 2 : 1) ars_kernel(const bdgfs_ars_args g)
 {
@@ -559,7 +560,8 @@ __global__ void __launch_bounds__(512, NA == 5 && AR <= 2 ? 2 : 1) ars_kernel(co
 // L_{q-1}) are reduced in the same launch when BDGFS_BDF_MOMN is set.  BQ > 0:
 // the order q at compile time (all 2 q rows of a chunk in flight); BQ = 0 reads
 // it from the arguments.  Moment algebra in one thread.  315 rows of 24^3 FP32,
-// Shakov, BDF-2: 86 -> 53 us on one B200 (512 threads a row).
+// Shakov, BDF-2, one B200: 86 -> 53 us (512 threads a row), 45 with a row per half
+// of them.  Bound: 116 registers leave one CTA an SM, so its barriers and loads show.
 template <typename T, int VEC, int NA, int BQ>
 __global__ void __launch_bounds__(512, NA == 5 ? 2 : 1) bdf_kernel(const bdgfs_bdf_args g)
 {

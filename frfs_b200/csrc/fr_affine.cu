@@ -15,10 +15,13 @@
 // FMAs a velocity and element instead of 2270.  Measured on one B200, 24^3 FP32
 // (bdgfs_fr_rhs_tensor -> this): RK stage of 210 hexes P2 593 -> 344 us (3.7 TB/s
 // of u, x1, x2 and out), L(u) of 128 quads P3 125 -> 61 us (3.7 TB/s).  Bound: the
-// latency of the dependent loads (u, three faces, x1, x2) at 16 warps an SM.
+// latency of the dependent loads (u, three faces, x1, x2) at 16 warps an SM (0.59 of
+// the copy rate), and instruction fetch of the unrolled body.
 //
 // A thread holds all solution points of an element at VB consecutive velocities
-// in registers: u, R and one direction's neighbours, loaded one direction ahead.
+// in registers: u, R and one direction's neighbours, loaded one direction ahead (FP32
+// hex P2 without spills; 284 bytes of them on hex P1 at four velocities, 548 on hex P2
+// in FP64).
 // Lanes choose their inflow face by a pointer select (two table entries a warp);
 // velocities of a chunk that disagree about the face take both.
 #include <algorithm>

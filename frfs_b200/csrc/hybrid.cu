@@ -214,9 +214,9 @@ struct OwnRow {
 // indicator_kernel with the row in shared memory: f is read once and the index and
 // coordinate work is per thread, not per chunk.  3001 rows of 24^3, one B200: 123 ->
 // 74 us (3.4 TB/s).  Four CTAs (36 warps) an SM; with the row in registers 96
-// registers leave two (121 us; 95 with the next row's copy in flight).  Bound: the
-// latency of the chain sums -> parameters -> deviation -> list entry at that occupancy,
-// and the FP32 -> FP64 conversions.  At 32^3 a row fills an SM's shared memory (one
+// registers leave two (121 us; 95 with the next row's copy in flight).  Bound: FP32 ->
+// FP64 conversions (their pipe is 55 % busy) and the barriers of the chain sums ->
+// parameters -> deviation -> list entry.  At 32^3 a row fills an SM's shared memory (one
 // CTA), so the streaming kernel stays.
 template <int N>
 __global__ void __launch_bounds__(OwnRow<N>::NT, OwnRow<N>::CTAS)
@@ -446,7 +446,9 @@ __global__ void __launch_bounds__(256) project_scatter_kernel(const bdgfs_hybrid
 }
 
 // project_scatter_kernel with the row in shared memory: Qc is read once.  3001 rows
-// of 24^3, one B200: 98 -> 64 us (5.2 TB/s; 84 with the row in registers).  Bound: HBM.
+// of 24^3, one B200: 98 -> 64 us (5.2 TB/s; 84 with the row in registers).  Bound: the
+// row's shared-memory traffic and FP32 <-> FP64 conversions (each about half busy);
+// HBM at 0.65 of the copy rate.
 template <int N>
 __global__ void __launch_bounds__(OwnRow<N>::NT, OwnRow<N>::CTAS)
     project_scatter_own_kernel(const bdgfs_hybrid_args h, const float* __restrict__ Qc, float* __restrict__ Q)

@@ -51,7 +51,8 @@ __device__ __forceinline__ void macro_store(const double (&m)[kMom], const Momen
 // line and keeps their four z-sums (f, cz f, cz^2 f, cz^3 f); the 13 moments
 // follow from those with 16 more multiply-adds per chunk, so an element costs
 // 4 + 16/VEC FP64 operations and one conversion instead of 13 and three 64-bit
-// index divisions.  Bound: the FP64 pipe and HBM (each row read once).  Measured
+// index divisions.  Bound: shared memory (the coordinates: 82 % of its wavefronts),
+// then the FP64 pipe (54 %) and HBM (each row read once: 0.63 of the copy rate).  Measured
 // with the fields formed in the same launch (they were some 30 small ones):
 // 5670 rows of 24^3 FP32 834 -> 74 us, 4.2 TB/s; 256 threads and one element
 // each was the form before.

@@ -19,8 +19,8 @@
 // 16^3, Nrho = 8, 6 directions, exact term, 144 distributions in FP64: 0.297 ->
 // 0.188 ms (the general variant with its second transform -> this one; error
 // against 64 bits unchanged); without the term 2048 in FP32: 2.21 -> 1.24 ms.
-// Bound: the FP64 pipe and the barriers between passes (FP64), shared memory
-// and the barriers (FP32).
+// Bound in FP64: shared memory (62 %, and its latency at eight warps an SM) and
+// the FP64 pipe (46 %).
 #pragma once
 #include "split.cuh"
 

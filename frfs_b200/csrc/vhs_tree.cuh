@@ -32,13 +32,12 @@
 // Work per radius at 12 directions: 2 + 6 passes of 312 pencil pairs and one of
 // 6 x 576, against 36 passes of 288 pairs, and 8 exchanges of a 120 KB cube
 // through shared memory against 24 of 110 KB.  Measured on one B200, Nrho = 12,
-// 12 directions: 2048 distributions 9.79 -> 6.09 ms (the variant with spectra
-// in tensor memory -> this one), 97 0.705 -> 0.358 ms, one 0.706 -> 0.085 ms
+// 12 directions: 2048 distributions 9.79 -> 5.98 ms (the variant with spectra
+// in tensor memory -> this one), 97 0.705 -> 0.350 ms, one 0.706 -> 0.084 ms
 // (radii cut over CTAs, split.cuh; so is the last, partly filled round of a long
-// list: 6.17 -> 6.09 ms for the 2048); the error against 64-bit arithmetic falls
-// from 4.5e-5 to 1e-5 of Q (fewer roundings into S_p).  Bound: the FP32 pipe (48 %
-// busy, 57 % on the sub-partitions with three warps) and the barriers of the
-// exchanges (shared memory 40 %).
+// list: 1.3 % of the 2048); the error against 64-bit arithmetic falls from 4.5e-5
+// to 1e-5 of Q (fewer roundings into S_p).  Bound: the FP32 pipe (51 % busy) and
+// the barriers of the exchanges, at 10 warps (shared memory 44 %).
 //
 // One CTA of 320 threads per distribution.  Thread t < 312 owns the pencil
 // (i, kz) = (t % 24, t / 24): ky in the x-passes, x in the y-passes.  Leaves:

@@ -10,10 +10,10 @@
 // two warps per lane quarter); those of kz = 16 sit in shared memory.  F, S_p and
 // G^ live in the CTA's scratch (L2), read and written by their own lanes only.
 //
-// 8 warps, so a thread may hold a 32-point pair (128 registers) and its S_p (32).
-// Measured on one B200, Nrho = 16, 12 directions: 501 distributions 15.4 -> 7.7 ms
-// (the warp-slab variant -> this one).  Bound: the FP32 pipe, with the barriers of
-// the y -> z exchange behind it.
+// 8 warps, so a thread may hold a 32-point pair (128 registers) beside what it works
+// with.  Measured on one B200, Nrho = 16, 12 directions: 501 distributions 15.4 ->
+// 7.87 ms (the warp-slab variant -> this one).  Bound: the latency of L2 (F, S_p and
+// half of the y -> z exchange) with 8 warps to hide it; the FP32 pipe is 33 % busy.
 #pragma once
 #include "vhs_tree.cuh"
 

@@ -19,10 +19,10 @@
 // group of eight rows.  G^ of both species stays in tensor memory.  F comes from
 // the CTA's scratch and the weights from their tables, through L2: 165 KB (like
 // pair) or 442 KB a slice.  Measured on one B200, Nrho = M = 12, 370 argon-krypton
-// pairs: 25.6 -> 10.5 ms (the general kernel of vss.cu -> this one; 12.3 ms before
-// the last round's distributions were cut over radii); error against 64-bit
-// arithmetic 4.0e-6 -> 3.5e-6 of Q.  Bound: the FP32 pipe and the barriers
-// between passes.  (The factors are real but for Nyquist terms; packing them as
+// pairs: 25.6 -> 10.3 ms (the general kernel of vss.cu -> this one; cutting the last
+// round's distributions over radii is 15 % of it); error against 64-bit arithmetic
+// 4.0e-6 -> 3.5e-6 to 3.7e-6 of Q.  Bound: shared memory (57 %), the FP32 pipe (48 %)
+// and the barriers between passes.  (The factors are real but for Nyquist terms; packing them as
 // one complex transform drops those terms, 1e-3 of Q on this mixture.)
 #include <algorithm>
 

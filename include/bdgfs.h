@@ -88,10 +88,12 @@ size_t bdgfs_vhs_scratch_bytes(const bdgfs_vhs_grid* grids, int32_t ngrids,
 
 /* Q for every distribution of every batch, in one persistent launch.
  * flags & BDGFS_PROJECT applies the FP64 minimal-norm conservation
- * projection Q <- Q - phi^T G^{-1} (phi Q); flags & BDGFS_EXACT runs a
- * second transform per (p, q) so that the result equals the reference's
- * complex-square form to rounding (2x the work).  work_counter: one device uint64 that this
- * call resets (stream-ordered) and uses to hand out distributions.
+ * projection Q <- Q - phi^T G^{-1} (phi Q); flags & BDGFS_EXACT adds the
+ * second-order Nyquist-plane term so that the result equals the reference's
+ * complex-square form to rounding (up to 2x the work).  work_counter: one device
+ * uint64 that this call resets (stream-ordered) and uses to hand out distributions.
+ * Should a bounded wait inside a kernel run out, the Q of the CTA it happened in
+ * are NaN (here and in bdgfs_vss_pair_collide).
  * Replaces DGFSVHSGLLScatteringModel.fs (frfs/solvers/dgfs/scattering.py:227)
  * called for every (elem, upt) by DGFSSystem.collide
  * (frfs/solvers/dgfs/system.py:199-218). */

@@ -3,9 +3,9 @@ threads (many rows), and rows without 16-byte alignment (one value per step,
 stage or order read from the arguments).  The 512-thread route is pinned to the
 reference's kernels and the oracle elsewhere.
 
-The routes run the same FP64 arithmetic with the row sums added in another
-order: n eps = 3e-12 of the sums' magnitudes (n = 24^3), which reach f through
-the targets; in FP32 the results round to neighbours at most (2^-23 each way,
+Few and many rows give the same bits.  Rows without alignment run the same FP64
+arithmetic with the row sums added in another order: n eps = 3e-12 of the sums'
+magnitudes (n = 24^3), which reach f through the targets; in FP32 the results round to neighbours at most (2^-23 each way,
 with dt nu < 1 no amplification): 3e-7."""
 import numpy as np
 import pytest
