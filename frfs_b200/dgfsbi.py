@@ -228,7 +228,7 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         self.d_sz = f64(vm.sz())
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == 'cuda' else 1
         self._nctas = nsm                              # CTAs that scratch is kept for
-        self._scratch = None
+        self._scratch, self._outgrown = None, []
         # FP64 conservation projection (species masses, total momentum and
         # energy); the reference's operator has none, so parity runs disable it
         self._project = self.cfg.getbool('scattering-model', 'conservation-projection', True)
@@ -282,18 +282,26 @@ class DGFSBiVSSGLLScatteringModel(DGFSBiScatteringModel):
         for p in (0, 1):
             a.f[p], a.Q[p] = fs[p].data_ptr(), Qs[p].data_ptr()
         nb = L.bdgfs_vss_pair_scratch_for(self._nctas, ndof, self.vm.Nrho())
-        if self._scratch is None or self._scratch.numel() < nb:
-            self._scratch = torch.empty(nb, dtype=torch.uint8, device=self.backend.device)
-        _lib.check(L.bdgfs_vss_pair_collide(C.byref(a), self._scratch.data_ptr(), nb, _lib.stream_ptr()),
+        scratch = self._at_least(nb, L.bdgfs_vss_pair_scratch_bytes(self._nctas))
+        _lib.check(L.bdgfs_vss_pair_collide(C.byref(a), scratch.data_ptr(), nb, _lib.stream_ptr()),
                    'bdgfs_vss_pair_collide')
+
+    def _at_least(self, nb, most):
+        """The scratch, grown to ``nb`` bytes (at least doubled, up to ``most``).  The
+        smaller ones it replaces are kept: a captured graph of an earlier call
+        holds their address.  Doubling bounds them by the last one's size."""
+        if self._scratch is None or self._scratch.numel() < nb:
+            if self._scratch is not None:
+                self._outgrown.append(self._scratch)
+                nb = max(nb, min(2 * self._scratch.numel(), most))
+            self._scratch = torch.empty(nb, dtype=torch.uint8, device=self.backend.device)
+        return self._scratch
 
     def _scratch_for(self, items):
         L = _lib.lib()
         nctas = max(1, min(self._nctas, items))
-        nb = L.bdgfs_vss_scratch_bytes(self.vm.Nv(), self.fp64, nctas)
-        if self._scratch is None or self._scratch.numel() < nb:
-            self._scratch = torch.empty(nb, dtype=torch.uint8, device=self.backend.device)
-        return self._scratch, nb
+        need = lambda k: L.bdgfs_vss_scratch_bytes(self.vm.Nv(), self.fp64, k)
+        return self._at_least(need(nctas), need(self._nctas)), need(nctas)
 
     def collide(self, fs, Qs, project=None):
         """Qs[p][dof] <- sum_q Q_pq(fs[p][dof], fs[q][dof]) for every
